@@ -154,7 +154,11 @@ __device__ __forceinline__ void process_strip_m(const DevParams& p, const float*
     const int W = p.W, H = p.H;
     const int y0 = rs * ROWS;
     if (y0 >= H) return; // warp-uniform
-    const int c0 = cw * 128 + lane * 4;
+    // a last strip of one lane would need halo cells on both its sides: it
+    // starts four columns early, which its first lane computes but does not
+    // write (the strip before it does)
+    const int lead = W - cw * 128 == 4 ? 4 : 0;
+    const int c0 = cw * 128 - lead + lane * 4;
     const bool active = c0 < W;
     const bool left_edge = lane == 0;
     const bool right_edge = active && (lane == 31 || c0 + 4 >= W);
@@ -230,7 +234,7 @@ __device__ __forceinline__ void process_strip_m(const DevParams& p, const float*
         }
         if (r < 2 * R) continue;
         const int y = y0 + r - 2 * R;
-        if (!active || y >= H) continue;
+        if (!active || y >= H || lane * 4 < lead) continue;
         float o[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {

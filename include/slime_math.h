@@ -122,6 +122,25 @@ SLM_FN uint32_t slm_f2u_bits(float x) { uint32_t u; memcpy(&u, &x, 4); return u;
 SLM_FN float slm_u2f_bits(uint32_t u) { float x; memcpy(&x, &u, 4); return x; }
 SLM_FN int slm_isnan(float x) { return x != x; }
 
+/* x / 9, correctly rounded, the shader's average of nine cells
+ * (compute.wgsl:185), without a division: Markstein's correction of a product
+ * with the rounded reciprocal (P. Markstein, "Computation of elementary
+ * functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1),
+ * 1990).  q = x * (1/9) is within an ulp of x / 9, its residual x - 9 q is
+ * exact as a fused multiply-add while nothing in it is subnormal or overflows,
+ * and q + residual * (1/9), rounded once, is x / 9 rounded.  slm_div9_ok says
+ * where that holds; the oracle's self-test compares every binary32 with the
+ * division. */
+SLM_FN int slm_div9_ok(float x) { /* 2^-100 <= x < 2^120, or +0 */
+    const uint32_t u = slm_f2u_bits(x);
+    return u - 0x0d800000u < 0x6e000000u || u == 0u;
+}
+SLM_FN float slm_div9_fast(float x) {
+    const float q = slm_mul(x, 0x1.c71c720000000p-4f); /* 1/9 rounded */
+    return slm_fma(slm_fma(-9.0f, q, x), 0x1.c71c720000000p-4f, q);
+}
+SLM_FN float slm_div9(float x) { return slm_div9_ok(x) ? slm_div9_fast(x) : slm_div(x, 9.0f); }
+
 /* WGSL min/max, pinned as IEEE 754-2019 minimumNumber/maximumNumber: a NaN
  * operand is ignored, and -0 orders below +0.  The device's fminf/fmaxf
  * (min.f32/max.f32) implement exactly this; the host spells it out. */

@@ -63,6 +63,7 @@ def lib():
         L.oracle_ph_window_mismatches.restype = C.c_uint64
         L.oracle_ph_finish_mismatches.argtypes = [C.c_uint32, C.c_uint32]
         L.oracle_ph_finish_mismatches.restype = C.c_uint64
+        L.oracle_div9_mismatches.restype = C.c_uint64
         L.oracle_jitter_hash.argtypes = [C.POINTER(C.c_int32), f32, f32, C.c_uint64, f32]
         L.oracle_uniform01.argtypes = [C.c_uint64, C.c_uint64, C.c_uint32, f32]
         L.oracle_gauss_weights.argtypes = [C.c_float, C.c_float, f32]
@@ -203,6 +204,12 @@ def ph_finish_mismatches(e_lo=139, e_hi=254):
     """Inputs with biased exponent e_lo..e_hi on which the 32-bit-word
     Payne-Hanek tail and its 64-bit statement disagree (0 expected)."""
     return int(lib().oracle_ph_finish_mismatches(e_lo, e_hi))
+
+
+def div9_mismatches():
+    """Inputs that slm_div9 takes without a division on which it differs from
+    the division (0 expected)."""
+    return int(lib().oracle_div9_mismatches())
 
 
 def sincos(x):

@@ -660,6 +660,17 @@ uint64_t oracle_ph_finish_mismatches(uint32_t e_lo, uint32_t e_hi) {
     }
     return bad;
 }
+/* Number of binary32 inputs slm_div9_ok accepts on which slm_div9_fast differs
+ * from the division by 9. */
+uint64_t oracle_div9_mismatches(void) {
+    uint64_t bad = 0;
+#pragma omp parallel for schedule(static) reduction(+ : bad)
+    for (int64_t i = 0; i < (1ll << 32); i++) {
+        const float x = slm_u2f_bits((uint32_t)i);
+        if (slm_div9_ok(x)) bad += slm_f2u_bits(slm_div9_fast(x)) != slm_f2u_bits(slm_div(x, 9.0f)) ? 1u : 0u;
+    }
+    return bad;
+}
 int oracle_gauss_weights(float radius, float sigma, float* w) {
     int R = slm_gauss_radius(radius, SLIME_MAX_BLUR_RADIUS);
     if (slm_gauss_weights(R, sigma, w) != 0) return -1;

@@ -312,6 +312,21 @@ __global__ void extra_deposits_kernel(const float* __restrict__ X, const float* 
     if ((unsigned)dx < (unsigned)W && (unsigned)dy < (unsigned)H) atomicAdd(counts + (size_t)dy * W + dx, m - 1);
 }
 
+// The deposits of the step that left these agents: one (or, in the
+// reference's dispatch, one per visit) at the cell of each agent's position,
+// the cell agent_move deposited at.
+__global__ void recount_kernel(const float* __restrict__ X, const float* __restrict__ Y,
+                               const uint32_t* __restrict__ ids, uint64_t n, int W, int H, uint32_t wy, uint32_t span,
+                               uint32_t* __restrict__ counts) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t m = wy ? slm_dispatch_visits_in(ids ? ids[i] : (uint32_t)i, wy, span) : 1u;
+    if (m == 0) return;
+    const int dx = slm_f2i(X[i]);
+    const int dy = slm_f2i(Y[i]);
+    if ((unsigned)dx < (unsigned)W && (unsigned)dy < (unsigned)H) atomicAdd(counts + (size_t)dy * W + dx, m);
+}
+
 template <int APT, int BS, int MINB, class Trail>
 cudaError_t launch_agents_persistent(const DevParams& p, const AgentsSoA& a, const Trail& trail, uint32_t* counts,
                                      uint8_t* marks, cudaStream_t s, const cudaAccessPolicyWindow* win, bool pdl) {
@@ -436,6 +451,14 @@ cudaError_t launch_agents(const DevParams& p, const AgentsSoA& a, const float* t
     case 15: return launch_agents_persistent<2, 256, 4>(p, a, tp, counts, marks, s, win, pdl);
     default: return launch_agents_variant<4, 256, 0>(p, a, tp, counts, marks, s, win, pdl);
     }
+}
+
+cudaError_t launch_recount(const DevParams& p, const AgentsSoA& a, uint32_t* counts, cudaStream_t s) {
+    if (a.n == 0) return cudaSuccess;
+    uint32_t wy = 0, span = 0;
+    if (p.dispatch_mode == SLIME_DISPATCH_REFERENCE) slm_dispatch_geometry(a.n, &wy, &span);
+    recount_kernel<<<blocks_for(a.n, 256), 256, 0, s>>>(a.x, a.y, a.ids, a.n, p.W, p.H, wy, span, counts);
+    return cudaGetLastError();
 }
 
 // A texture over trail buffer `t` (W x H binary32, row pitch 4W bytes) for

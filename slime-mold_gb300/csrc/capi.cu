@@ -396,6 +396,20 @@ bool trail_window(const slime_ctx* ctx, const float* t, cudaAccessPolicyWindow* 
     return true;
 }
 
+// The trail tile and the agent-kernel shape the next steps use: the option's,
+// else the autotuner's, else the default for these parameters.
+void choose_kernels(slime_ctx* ctx) {
+    const bool marks = ctx->dev.dep >= 1.0f && ctx->agents.n <= (uint64_t)ctx->W * ctx->H;
+    const int tile = ctx->opt.trail_tile ? (int)ctx->opt.trail_tile - 1
+                                         : (ctx->tuned_tile >= 0 ? ctx->tuned_tile : trail_tile_default(ctx->dev, marks));
+    const int shape = ctx->opt.agent_shape ? (int)ctx->opt.agent_shape - 1 : (ctx->tuned_shape >= 0 ? ctx->tuned_shape : 0);
+    if (tile != ctx->tile || shape != ctx->agent_shape) {
+        ctx->tile = tile;
+        ctx->agent_shape = shape;
+        invalidate_graphs(ctx);
+    }
+}
+
 // Whether a step keeps a clean trail clean (finite values >= 0, or +inf):
 // the subtractive decay never raises a value, the multiplicative one with a
 // factor in [0, 1] neither; the fold, the blur's non-negative weights and the
@@ -411,15 +425,34 @@ bool keeps_trail_clean(const DevParams& d) {
 // fold of k deposits depends only on whether k > 0: one byte per cell carries
 // it, written with plain stores instead of 32-bit atomics, and the trail pass
 // reads 1 byte per cell instead of 4 and clears 1 instead of 4.  The result
-// is the same, bit for bit.  The host decides, from the parameters, the tile
-// (the streaming tiles read marks) and what it knows of the trail: clean
-// after creation, clear and resize, checked on upload, kept by steps that
-// keep it (keeps_trail_clean).
+// is the same, bit for bit.  The host decides, from the parameters and what
+// it knows of the trail: clean after creation, clear and resize, checked on
+// upload, kept by steps that keep it (keeps_trail_clean).
 bool marks_allowed(const slime_ctx* ctx) {
     if (ctx->opt.exact_counts || ctx->agents.n == 0 || !ctx->trail_clean) return false;
     return ctx->dev.dep >= 1.0f && keeps_trail_clean(ctx->dev);
 }
-bool use_marks(const slime_ctx* ctx) { return marks_allowed(ctx) && trail_tile_streams(ctx->dev, ctx->tile); }
+// Marks where there is at most one agent per cell: four cells share a mark
+// word, so agents that crowd together OR the same word, which the L2 does one
+// after another, while the trail pass saves 6 bytes a cell.  Agent and trail
+// pass after 1000 steps in Morton order, marks / counts: one agent per cell
+// (4096^2) 214 + 28 / 204 + 43 us, seven (10 M on 1600x900) 159 + 6 / 134 + 8.
+bool use_marks(const slime_ctx* ctx) {
+    return marks_allowed(ctx) && ctx->agents.n <= (uint64_t)ctx->W * ctx->H;
+}
+
+// The counts of a step that recorded marks, made from the agents it left:
+// when they are asked for, and before the agents change.
+int make_counts(slime_ctx* ctx) {
+    if (!ctx->last_counts_valid || !ctx->last_marks || ctx->last_no_counts) return SLIME_OK;
+    const int last = 1 - ctx->cur;
+    CK(cudaMemsetAsync(ctx->counts[last], 0, (size_t)ctx->W * ctx->H * sizeof(uint32_t), ctx->stream),
+       "clearing deposit counts");
+    CK(launch_recount(ctx->last_dev, ctx->agents, ctx->counts[last], ctx->stream), "counting deposits");
+    ctx->counts_dirty[last] = true;
+    ctx->last_marks = false;
+    return SLIME_OK;
+}
 
 // The record the next step writes (counts[cur] or marks[cur]) must start at
 // zero; a record left behind by steps of the other kind is cleared here,
@@ -445,8 +478,12 @@ void after_steps(slime_ctx* ctx, bool marks, uint32_t m) {
     bool* dirty = marks ? ctx->marks_dirty : ctx->counts_dirty;
     dirty[ctx->cur] = false;
     dirty[1 - ctx->cur] = true;
+    const bool no_counts = marks_allowed(ctx) && (ctx->opt.trail_tile || ctx->tuned_tile >= 0) &&
+                           trail_tile_streams(ctx->dev, ctx->tile);
     ctx->trail_clean = ctx->trail_clean && keeps_trail_clean(ctx->dev);
     ctx->last_marks = marks;
+    ctx->last_no_counts = no_counts;
+    ctx->last_dev = ctx->dev;
     ctx->last_counts_valid = true;
 }
 
@@ -475,11 +512,12 @@ cudaError_t enqueue_trail_pass(slime_ctx* ctx, bool marks, bool pdl) {
 }
 
 // `chained`: the operation before this step on the stream is the previous
-// step's trail pass, so the agent pass may start while it finishes; the trail
-// pass always follows the agent pass's kernel when there are agents.
+// step's trail pass, so the agent pass may start while it finishes (not behind
+// the shared-memory tiles, see trail_tile.cuh); the trail pass always follows
+// the agent pass's kernel when there are agents.
 cudaError_t enqueue_step(slime_ctx* ctx, bool marks, bool chained) {
     const bool agents = ctx->agents.n > 0;
-    cudaError_t e = enqueue_agents_pass(ctx, marks, chained && agents);
+    cudaError_t e = enqueue_agents_pass(ctx, marks, chained && agents && trail_tile_streams(ctx->dev, ctx->tile));
     if (e != cudaSuccess) return e;
     e = enqueue_trail_pass(ctx, marks, agents);
     if (e != cudaSuccess) return e;
@@ -743,7 +781,6 @@ slime_ctx* slime_create(uint32_t width, uint32_t height, uint64_t n_agents, int*
     ctx->opt.reorder_cell_log2 = 2;
     ctx->opt.l2_persist = 1;
     ctx->opt.trail_tile = 0;
-    ctx->tile = trail_tile_default();
     int rc = SLIME_OK;
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) {
         rc = SLIME_ERR_CUDA;
@@ -753,7 +790,9 @@ slime_ctx* slime_create(uint32_t width, uint32_t height, uint64_t n_agents, int*
         slime_params_from_settings(&s, width, height, &ctx->params);
         const char* why = nullptr;
         if (!make_dev_params(ctx->params, width, height, &ctx->dev, &why)) rc = SLIME_ERR_INVALID_ARGUMENT;
-        else if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = SLIME_ERR_CUDA;
+        choose_kernels(ctx);
+        if (rc != SLIME_OK) {
+        } else if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = SLIME_ERR_CUDA;
         else setup_l2(ctx);
     }
     if (rc != SLIME_OK) {
@@ -805,6 +844,7 @@ int slime_set_params(slime_ctx* ctx, const SlimeParams* params) {
     if (memcmp(&d, &ctx->dev, sizeof d) != 0) {
         ctx->dev = d;
         invalidate_graphs(ctx); // the parameter block is baked into the captured launches
+        choose_kernels(ctx);
     }
     return SLIME_OK;
 }
@@ -834,13 +874,7 @@ int slime_set_options(slime_ctx* ctx, const SlimeOptions* o) {
         setup_l2(ctx);
         invalidate_graphs(ctx);
     }
-    int tile = o->trail_tile ? (int)o->trail_tile - 1 : (ctx->tuned_tile >= 0 ? ctx->tuned_tile : trail_tile_default());
-    int shape = o->agent_shape ? (int)o->agent_shape - 1 : (ctx->tuned_shape >= 0 ? ctx->tuned_shape : 0);
-    if (tile != ctx->tile || shape != ctx->agent_shape) {
-        ctx->tile = tile;
-        ctx->agent_shape = shape;
-        invalidate_graphs(ctx);
-    }
+    choose_kernels(ctx);
     return SLIME_OK;
 }
 
@@ -876,6 +910,7 @@ int slime_upload_agents(slime_ctx* ctx, const float* aos, uint64_t n) {
                          (unsigned long long)n, (unsigned long long)ctx->agents.n);
     if (n == 0) return SLIME_OK;
     int rc;
+    if ((rc = make_counts(ctx)) != SLIME_OK) return rc;
     if ((rc = ensure_staging(ctx, n * sizeof(float4))) != SLIME_OK) return rc;
     CK(cudaMemcpyAsync(ctx->staging, aos, n * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream), "uploading agents");
     CK(launch_aos_to_soa((const float4*)ctx->staging, ctx->agents, ctx->stream), "converting agents");
@@ -902,10 +937,11 @@ int slime_download_agents(slime_ctx* ctx, float* aos, uint64_t n) {
 int slime_seed_agents(slime_ctx* ctx, uint64_t seed, float hmin, float hmax) {
     if (!ctx || !isfinite(hmin) || !isfinite(hmax)) return SLIME_ERR_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
+    int rc = make_counts(ctx);
+    if (rc != SLIME_OK) return rc;
     CK(launch_seed_agents(ctx->agents, seed, (float)ctx->W, (float)ctx->H, hmin, hmax, ctx->params.agent_speed_min,
                           ctx->params.agent_speed_max, ctx->stream),
        "seeding agents");
-    int rc;
     if ((rc = reset_ids(ctx)) != SLIME_OK) return rc;
     CK(cudaStreamSynchronize(ctx->stream), "seeding agents");
     return SLIME_OK;
@@ -984,6 +1020,7 @@ int slime_resize(slime_ctx* ctx, uint32_t width, uint32_t height) {
     ctx->params = np;
     ctx->dev = d;
     ctx->tuned_tile = -1;
+    choose_kernels(ctx);
     ctx->l2_tuned_off = false;
     ctx->l2_window_passes = 3;
     setup_l2(ctx);
@@ -997,12 +1034,14 @@ int slime_set_agent_count(slime_ctx* ctx, uint64_t n, uint64_t seed) {
     cudaSetDevice(ctx->device);
     int rc;
     if ((rc = valid_size(ctx->err, ctx->W, ctx->H, n)) != SLIME_OK) return rc;
+    if ((rc = make_counts(ctx)) != SLIME_OK) return rc;
     CK(cudaStreamSynchronize(ctx->stream), "changing the agent count");
     // the new block replaces the agents only once allocated: out of memory,
     // the context keeps its agents
     invalidate_graphs(ctx);
     free_adjoint(ctx);
     if ((rc = alloc_agents(ctx, n)) != SLIME_OK) return rc;
+    choose_kernels(ctx);
     ctx->reordered = false;
     // src/main.rs:700-712 draws x, y, angle in [0, 2*pi) and speed anew.
     return slime_seed_agents(ctx, seed, 0.0f, 6.28318530718f);
@@ -1193,10 +1232,12 @@ int slime_download_deposit_counts(slime_ctx* ctx, uint32_t* counts, uint64_t n_c
         memset(counts, 0, n_cells * sizeof(uint32_t));
         return SLIME_OK;
     }
-    if (ctx->last_marks)
+    if (ctx->last_no_counts)
         return set_error(ctx->err, SLIME_ERR_STATE,
                          "the last step recorded which cells received deposits, not how many (every deposit "
                          "saturated the fold); set options.exact_counts = 1 to keep counts");
+    const int rc = make_counts(ctx);
+    if (rc != SLIME_OK) return rc;
     CK(cudaMemcpyAsync(counts, ctx->counts[1 - ctx->cur], n_cells * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                        ctx->stream),
        "downloading deposit counts");
@@ -1298,13 +1339,12 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
     // 1. trail tiles.  The trial launches read trail[cur] and the (zero)
     // counts[cur] and write the other buffers, so the state is untouched; the
     // previous step's counts are overwritten with zeros.
-    // Each tile runs with the deposit record the steps would use with it.
+    // Each tile runs with the deposit record the steps would use.
     float best = 1e30f;
     int best_tile = ctx->tile;
-    const bool marks_ok = marks_allowed(ctx);
+    const bool mk = use_marks(ctx);
     for (int t = 0; t < trail_tile_count(); t++) {
         if (!trail_tile_supported(ctx->dev, t) || (t == kTrailTileTma && !ctx->tmaps.ok)) continue;
-        const bool mk = marks_ok && trail_tile_streams(ctx->dev, t);
         auto trial = [&]() {
             return mk ? launch_trail_marks(ctx->dev, t, ctx->trail[cur], ctx->marks[cur], ctx->trail[1 - cur],
                                            ctx->marks[1 - cur], ctx->stream, nullptr, false, &ctx->tmaps, cur)
@@ -1339,8 +1379,7 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
     }
     int best_shape = ctx->agent_shape;
     if (ctx->agents.n > 0) {
-        const int tile_now = ctx->opt.trail_tile ? (int)ctx->opt.trail_tile - 1 : best_tile;
-        uint8_t* mk = (marks_ok && trail_tile_streams(ctx->dev, tile_now)) ? ctx->marks[cur] : nullptr;
+        uint8_t* marks = mk ? ctx->marks[cur] : nullptr;
         const size_t abytes = 4 * ctx->agents.n_pad * sizeof(float);
         void* snap = nullptr;
         if (dev_alloc((void**)&snap, abytes) == cudaSuccess) {
@@ -1352,16 +1391,16 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
                     if (agent_shape_uses_texture(sh) && !ctx->trail_tex[cur]) continue;
                     cudaMemcpyAsync(ctx->agent_block, snap, abytes, cudaMemcpyDeviceToDevice, ctx->stream);
                     launch_agents(ctx->dev, ctx->agents, ctx->trail[cur], ctx->counts[cur], ctx->stream, sh, nullptr,
-                                  ctx->trail_tex[cur], mk);
+                                  ctx->trail_tex[cur], marks);
                     cudaEventRecord(e0, ctx->stream);
                     for (uint32_t r = 0; r < reps; r++)
                         launch_agents(ctx->dev, ctx->agents, ctx->trail[cur], ctx->counts[cur], ctx->stream, sh,
-                                      nullptr, ctx->trail_tex[cur], mk);
+                                      nullptr, ctx->trail_tex[cur], marks);
                     cudaEventRecord(e1, ctx->stream);
                     CK(cudaEventSynchronize(e1), "autotuning");
                     float ms = 0;
                     cudaEventElapsedTime(&ms, e0, e1);
-                    ctx->launches += (reps + 1) * (uint64_t)agent_pass_kernels(ctx->dev, ctx->agents.n, mk != nullptr);
+                    ctx->launches += (reps + 1) * (uint64_t)agent_pass_kernels(ctx->dev, ctx->agents.n, mk);
                     if (ms < best_a) {
                         best_a = ms;
                         best_shape = sh;
@@ -1381,13 +1420,7 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
     ctx->last_counts_valid = false;
     ctx->tuned_tile = best_tile;
     ctx->tuned_shape = best_shape;
-    int tile = ctx->opt.trail_tile ? (int)ctx->opt.trail_tile - 1 : best_tile;
-    int shape = ctx->opt.agent_shape ? (int)ctx->opt.agent_shape - 1 : best_shape;
-    if (tile != ctx->tile || shape != ctx->agent_shape) {
-        ctx->tile = tile;
-        ctx->agent_shape = shape;
-        invalidate_graphs(ctx);
-    }
+    choose_kernels(ctx);
     // 3. the persisting-L2 window, with the tile and shape just chosen
     if (ctx->opt.l2_persist && ctx->agents.n > 0) {
         ctx->l2_tuned_off = false;

@@ -128,6 +128,20 @@ __device__ __forceinline__ float apply_decay_m(const DevParams& p, float v) {
     return kMode == (int)SLIME_DECAY_MULTIPLY ? slm_mul(v, p.decay) : slm_max(slm_sub(v, p.decay_k), 0.0f);
 }
 
+// Four box sums divided by 9 (slm_div9 of each): one range test for the four.
+__device__ __noinline__ static float4 div9x4_general(float a, float b, float c, float d) {
+    return make_float4(slm_div9(a), slm_div9(b), slm_div9(c), slm_div9(d));
+}
+__device__ __forceinline__ void slm_div9x4(float* v) {
+    if (slm_div9_ok(v[0]) && slm_div9_ok(v[1]) && slm_div9_ok(v[2]) && slm_div9_ok(v[3])) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = slm_div9_fast(v[j]);
+    } else {
+        const float4 r = div9x4_general(v[0], v[1], v[2], v[3]);
+        v[0] = r.x, v[1] = r.y, v[2] = r.z, v[3] = r.w;
+    }
+}
+
 // Wrap g into [0, n) for g in [-n*k, n*(k+1)); the loops run at most once for
 // the halos the kernels use unless the grid is smaller than the blur radius.
 __device__ __forceinline__ int wrap_coord(int g, int n) {

@@ -37,6 +37,11 @@ struct slime_ctx {
     bool marks_dirty[2] = {false, false};
     bool trail_clean = true; // every value of trail[cur] is finite and >= 0 (or +inf)
     bool last_marks = false; // the last step recorded marks, not counts
+    // its deposits all saturated the fold, on a streaming tile that was chosen or
+    // tuned for: no counts download after it.  After other steps that recorded
+    // marks the counts are made on demand.
+    bool last_no_counts = false;
+    slime::DevParams last_dev{}; // the parameters it ran with
 
     SlimeParams params{};
     slime::DevParams dev{};
@@ -115,8 +120,9 @@ namespace slime {
 int set_error(std::string& err, int code, const char* fmt, ...);
 int cuda_error(std::string& err, cudaError_t e, const char* what);
 void invalidate_graphs(slime_ctx* ctx);
-bool marks_allowed(const slime_ctx* ctx);
+void choose_kernels(slime_ctx* ctx);
 bool keeps_trail_clean(const DevParams& d);
+bool marks_allowed(const slime_ctx* ctx);
 bool use_marks(const slime_ctx* ctx);
 int prepare_deposits(slime_ctx* ctx, bool marks);
 cudaError_t enqueue_step(slime_ctx* ctx, bool marks, bool chained);

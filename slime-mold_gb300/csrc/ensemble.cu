@@ -606,9 +606,10 @@ int check_barrier(slime_ensemble* e) {
 // Whether colony c records its deposits as byte marks in the next steps:
 // the lanes engine on a streaming trail tile, a deposition of at least 1 on
 // a clean trail that the colony's steps keep clean (every deposit then folds
-// the cell to 1, so whether a cell received any carries the fold).
+// the cell to 1, so whether a cell received any carries the fold), and at most
+// one agent per cell (use_marks in capi.cu).
 bool colony_marks(const slime_ensemble* e, const Colony& c) {
-    return e->engine == SLIME_ENSEMBLE_LANES && c.n > 0 && c.trail_clean && c.dev.dep >= 1.0f &&
+    return e->engine == SLIME_ENSEMBLE_LANES && c.n > 0 && c.n <= (uint64_t)c.W * c.H && c.trail_clean && c.dev.dep >= 1.0f &&
            keeps_trail_clean(c.dev) && trail_tile_streams(c.dev, e->lane_trail_tile);
 }
 

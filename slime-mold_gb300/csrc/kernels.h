@@ -50,6 +50,9 @@ cudaError_t launch_agents(const DevParams& p, const AgentsSoA& a, const float* t
 int agent_pass_kernels(const DevParams& p, uint64_t n, bool marks);
 // How many agents (ids 0 .. this - 1) the reference's dispatch updates.
 uint64_t reference_dispatch_updated(uint64_t n);
+// Adds to `counts` the deposits the last step made, from the agents it left
+// (an agent deposits at the cell it moves to).
+cudaError_t launch_recount(const DevParams& p, const AgentsSoA& a, uint32_t* counts, cudaStream_t s);
 cudaTextureObject_t make_trail_texture(const float* trail, uint32_t W, uint32_t H);
 // AoS staging (x, y, angle, speed per agent, id order) <-> SoA slots.
 cudaError_t launch_aos_to_soa(const float4* aos, const AgentsSoA& a, cudaStream_t s);
@@ -66,7 +69,10 @@ struct TrailTile {
 };
 int trail_tile_count();
 TrailTile trail_tile(int index);
-int trail_tile_default();
+// The tile of a context that neither chose nor tuned one, for steps that record
+// marks or counts; with `aligned` false one that reads and writes buffers of
+// any alignment.
+int trail_tile_default(const DevParams& p, bool marks, bool aligned = true);
 // Whether tile `index` can run this parameter set / grid (the streaming
 // tiles need W % 4 == 0 and a blur radius of 1 or 2).
 bool trail_tile_supported(const DevParams& p, int tile);
@@ -82,19 +88,19 @@ constexpr int kTrailTileTma = 10;
 
 // Fused trail pass: out = Diffuse(Decay(Fold(in, counts_in))); zeroes
 // counts_zero (the other step's count buffer, may be null) over the same cells.
-// With `pdl` a streaming tile launches as a programmatic dependent of the
-// kernel before it in the stream (the agent pass); the shared-memory tiles
-// always launch in order.
+// With `pdl` a streaming or tensor-copy tile launches as a programmatic
+// dependent of the kernel before it in the stream (the agent pass); the
+// shared-memory tiles always launch in order.  A tile that cannot run this
+// parameter set gives way to the default one.
 // The tensor-copy tile needs `maps` over the context's buffers and the index
 // `cur` of the buffers `in`/`counts_in` are.
 cudaError_t launch_trail(const DevParams& p, int tile, const float* in, const uint32_t* counts_in, float* out,
                          uint32_t* counts_zero, cudaStream_t s, const cudaAccessPolicyWindow* win = nullptr,
                          bool pdl = false, const TrailMaps* maps = nullptr, int cur = 0);
-// Whether tile `index` is a streaming tile that runs here (the only ones that
-// read deposit marks).
+// Whether tile `index` is a streaming or tensor-copy tile that runs here.
 bool trail_tile_streams(const DevParams& p, int tile);
 // The same pass folding per-cell byte marks (0/1) instead of counts; zeroes
-// marks_zero.  Streaming tiles only (cudaErrorInvalidValue otherwise).
+// marks_zero.
 cudaError_t launch_trail_marks(const DevParams& p, int tile, const float* in, const uint8_t* marks_in, float* out,
                                uint8_t* marks_zero, cudaStream_t s, const cudaAccessPolicyWindow* win = nullptr,
                                bool pdl = false, const TrailMaps* maps = nullptr, int cur = 0);

@@ -69,10 +69,12 @@ int step_with_counts(const SlimeParams* params, uint32_t width, uint32_t height,
     a.n = n_agents;
     a.n_pad = n_agents;
     // One agent per thread (scalar loads need no padding or 16-byte
-    // alignment of the caller's arrays) and the shared-memory trail tile.
+    // alignment of the caller's arrays); the trail pass of unaligned trails or
+    // counts is a shared-memory tile.
     const int kScalarShape = 2;
     cudaError_t e = launch_agents(d, a, d_trail_in, counts, s, kScalarShape, nullptr);
-    if (e == cudaSuccess) e = launch_trail(d, trail_tile_default(), d_trail_in, counts, d_trail_out, nullptr, s, nullptr);
+    const bool aligned = (((uintptr_t)d_trail_in | (uintptr_t)d_trail_out | (uintptr_t)counts) & 15) == 0;
+    if (e == cudaSuccess) e = launch_trail(d, trail_tile_default(d, false, aligned), d_trail_in, counts, d_trail_out, nullptr, s, nullptr);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return SLIME_ERR_CUDA;

@@ -2,12 +2,13 @@
 //
 // The reference runs decay_trail (compute.wgsl:148-161) and diffuse_trail
 // (compute.wgsl:164-195) as two full passes over the trail, the blur in place.
-// Here one kernel reads the pre-step trail and the step's deposit counts once
-// (tile plus halo staged in shared memory), applies the sequential deposit
-// fold and the decay while staging, blurs from shared memory, writes the new
-// trail to the other buffer and zeroes the other step's count buffer.
-// HBM traffic per cell: 4 B trail in + 4 B counts in + 4 B trail out +
-// 4 B counts zeroed; halo re-reads hit L2.
+// Here one kernel reads the pre-step trail and the step's deposit record once,
+// applies the sequential deposit fold and the decay, blurs, writes the new
+// trail to the other buffer and zeroes the other step's record: rows streamed
+// through registers (trail_stream.cuh), tiles staged in shared memory
+// (trail_tile.cuh) or by tensor copies (trail_tma.cu).
+// HBM traffic per cell: 4 B trail in + 4 B out, and 4 B read + 4 B zeroed of
+// counts or 1 B + 1 B of marks; halo re-reads hit L2.
 //
 // Box mode sums the nine taps in the shader's order (dy outer, dx inner,
 // starting from 0.0) and divides by 9.0, so it matches the shader's arithmetic
@@ -15,93 +16,10 @@
 // multiply-adds over taps -R..R).
 #include "kernels.h"
 #include "trail_stream.cuh"
+#include "trail_tile.cuh"
 
 namespace slime {
 namespace {
-
-constexpr int kThreads = 256;
-
-template <int TW, int TH, int R>
-__device__ __forceinline__ void stage_tile(const DevParams& p, const float* __restrict__ in,
-                                           const uint32_t* __restrict__ cin, float* s, int x0, int y0) {
-    constexpr int SW = TW + 2 * R, SH = TH + 2 * R;
-    const int W = p.W, H = p.H;
-    for (int i = threadIdx.x; i < SH * SW; i += kThreads) {
-        int ly = i / SW;
-        int lx = i - ly * SW;
-        int gx = wrap_coord(x0 + lx - R, W);
-        int gy = wrap_coord(y0 + ly - R, H);
-        int gi = gy * W + gx;
-        float v = fold_deposits(__ldg(in + gi), __ldg(cin + gi), p.dep);
-        s[i] = apply_decay(p, v);
-    }
-}
-
-template <int TW, int TH>
-__global__ void __launch_bounds__(kThreads) trail_box3_kernel(const __grid_constant__ DevParams p,
-                                                              const float* __restrict__ in,
-                                                              const uint32_t* __restrict__ cin,
-                                                              float* __restrict__ out,
-                                                              uint32_t* __restrict__ czero) {
-    constexpr int R = 1, SW = TW + 2 * R;
-    extern __shared__ float smem[];
-    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
-    stage_tile<TW, TH, R>(p, in, cin, smem, x0, y0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < TW * TH; i += kThreads) {
-        int ly = i / TW;
-        int lx = i - ly * TW;
-        int gx = x0 + lx, gy = y0 + ly;
-        if (gx >= p.W || gy >= p.H) continue;
-        const float* c = smem + (ly + 1) * SW + (lx + 1);
-        float sum = 0.0f;
-#pragma unroll
-        for (int dy = -1; dy <= 1; dy++)
-#pragma unroll
-            for (int dx = -1; dx <= 1; dx++) sum = slm_add(sum, c[dy * SW + dx]);
-        float avg = slm_div(sum, 9.0f);
-        int gi = gy * p.W + gx;
-        out[gi] = slm_mix(c[0], avg, p.rate);
-        if (czero) czero[gi] = 0u;
-    }
-}
-
-template <int TW, int TH, int R>
-__global__ void __launch_bounds__(kThreads) trail_gauss_kernel(const __grid_constant__ DevParams p,
-                                                               const float* __restrict__ in,
-                                                               const uint32_t* __restrict__ cin,
-                                                               float* __restrict__ out,
-                                                               uint32_t* __restrict__ czero) {
-    constexpr int SW = TW + 2 * R, SH = TH + 2 * R;
-    extern __shared__ float smem[];
-    float* s = smem;
-    float* h = smem + SH * SW;
-    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
-    stage_tile<TW, TH, R>(p, in, cin, s, x0, y0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < SH * TW; i += kThreads) {
-        int ly = i / TW;
-        int lx = i - ly * TW;
-        const float* row = s + ly * SW + lx;
-        float acc = 0.0f;
-#pragma unroll
-        for (int t = 0; t <= 2 * R; t++) acc = slm_fma(p.w[t], row[t], acc);
-        h[i] = acc;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < TW * TH; i += kThreads) {
-        int ly = i / TW;
-        int lx = i - ly * TW;
-        int gx = x0 + lx, gy = y0 + ly;
-        if (gx >= p.W || gy >= p.H) continue;
-        float acc = 0.0f;
-#pragma unroll
-        for (int t = 0; t <= 2 * R; t++) acc = slm_fma(p.w[t], h[(ly + t) * TW + lx], acc);
-        int gi = gy * p.W + gx;
-        out[gi] = slm_mix(s[(ly + R) * SW + lx + R], acc, p.rate);
-        if (czero) czero[gi] = 0u;
-    }
-}
 
 template <int R, bool kGauss, int ROWS, class D>
 __global__ void __launch_bounds__(128) trail_stream_kernel(const __grid_constant__ DevParams p,
@@ -133,51 +51,19 @@ cudaError_t launch_stream_rows(const DevParams& p, const float* in, const D* cin
     return launch_stream<2, true, ROWS, D>(p, in, cin, out, cz, s, win, pdl);
 }
 
-const TrailTile kTiles[] = {{32, 8}, {64, 8}, {32, 16}, {64, 16}, {128, 8}, {128, 16}, {256, 8}};
+const TrailTile kTiles[] = {{64, 8}, {64, 16}, {64, 32}, {128, 8}, {128, 16}, {128, 32}, {128, 64}};
 constexpr int kNumTiles = (int)(sizeof(kTiles) / sizeof(kTiles[0]));
 
-template <int TW, int TH>
-cudaError_t launch_tile(const DevParams& p, const float* in, const uint32_t* cin, float* out, uint32_t* cz,
-                        cudaStream_t s, const cudaAccessPolicyWindow* win) {
-    dim3 grid((p.W + TW - 1) / TW, (p.H + TH - 1) / TH);
-    if (p.blur_mode == SLIME_BLUR_GAUSS && p.R > 0) {
-        size_t smem;
-#define SLIME_GAUSS_CASE(RR)                                                                                 \
-    case RR:                                                                                                 \
-        smem = sizeof(float) * ((TH + 2 * RR) * (TW + 2 * RR) + (TH + 2 * RR) * TW);                         \
-        if (smem > 48 * 1024) {                                                                              \
-            cudaError_t e = cudaFuncSetAttribute(trail_gauss_kernel<TW, TH, RR>,                             \
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
-            if (e != cudaSuccess) return e;                                                                  \
-        }                                                                                                    \
-        {                                                                                                    \
-            cudaError_t le = launch_k(trail_gauss_kernel<TW, TH, RR>, grid, dim3(kThreads), smem, s, win, p, in,  \
-                                      cin, out, cz);                                                         \
-            if (le != cudaSuccess) return le;                                                                \
-        }                                                                                                    \
-        break;
-        switch (p.R) {
-            SLIME_GAUSS_CASE(1)
-            SLIME_GAUSS_CASE(2)
-            SLIME_GAUSS_CASE(3)
-            SLIME_GAUSS_CASE(4)
-            SLIME_GAUSS_CASE(5)
-            SLIME_GAUSS_CASE(6)
-            SLIME_GAUSS_CASE(7)
-            SLIME_GAUSS_CASE(8)
-        default:
-            return cudaErrorInvalidValue;
-        }
-#undef SLIME_GAUSS_CASE
-    } else if (p.blur_mode == SLIME_BLUR_GAUSS) {
-        // Radius 0: the blur is the identity; weights are {1}.
-        size_t smem = sizeof(float) * (TH * TW + TH * TW);
-        return launch_k(trail_gauss_kernel<TW, TH, 0>, grid, dim3(kThreads), smem, s, win, p, in, cin, out, cz);
-    } else {
-        size_t smem = sizeof(float) * (TH + 2) * (TW + 2);
-        return launch_k(trail_box3_kernel<TW, TH>, grid, dim3(kThreads), smem, s, win, p, in, cin, out, cz);
+cudaError_t launch_tile_index(int tile, SLIME_TILE_ARGS) {
+    switch (tile) {
+    case 0: return launch_tile_64x8(p, in, counts, marks, o, s, win);
+    case 1: return launch_tile_64x16(p, in, counts, marks, o, s, win);
+    case 2: return launch_tile_64x32(p, in, counts, marks, o, s, win);
+    case 3: return launch_tile_128x8(p, in, counts, marks, o, s, win);
+    case 4: return launch_tile_128x16(p, in, counts, marks, o, s, win);
+    case 5: return launch_tile_128x32(p, in, counts, marks, o, s, win);
+    default: return launch_tile_128x64(p, in, counts, marks, o, s, win);
     }
-    return cudaGetLastError();
 }
 
 } // namespace
@@ -193,7 +79,25 @@ TrailTile trail_tile(int index) {
     if (index >= kNumTiles && index < kNumTiles + kNumStream) return TrailTile{128, 8 << (index - kNumTiles)};
     return kTiles[(index >= 0 && index < kNumTiles) ? index : 0];
 }
-int trail_tile_default() { return 3; }
+// Measured as whole steps of one agent (us; tile 4 = 128 x 16, 5 = 128 x 32,
+// 7 = 8-row strips), each side of the lines drawn here:
+//   box, tile 4 / 5 / 7: 512^2 4.0 / 4.5 / 4.8, 1600x900 5.6 / 5.7 / 6.2,
+//     2048^2 11.3 / 9.7 / 9.8, 4096^2 42.7 / 37.5 / 32.7 (the strips walk
+//     their rows one after another, which only a large grid hides);
+//   Gaussian radius 1, marks, 4 / 7: 512^2 4.0 / 3.7, 2048^2 10.9 / 7.3;
+//     counts (four times the registers a row): 512^2 4.4 / 6.1,
+//     1600x900 6.4 / 6.5, 2048^2 12.5 / 9.9;
+//   what strips cannot run, 4 / 5: radius 5 1600x900 7.5 / 7.3, 2048^2
+//     15.5 / 13.1; radius 1 3001x2003 18.9 / 20.9, radius 2 19.9 / 17.9.
+// (The 64 x 16 tile of one cell per thread that was the default before took
+// 6.6 and 14.4 for the two smallest boxes, 43.6 for radius 5 at 2048^2.)
+int trail_tile_default(const DevParams& p, bool marks, bool aligned) {
+    const int64_t cells = (int64_t)p.W * p.H;
+    const bool gauss = p.blur_mode == SLIME_BLUR_GAUSS;
+    const int64_t strips_from = gauss ? (marks ? 0 : 2000000) : 6000000;
+    if (aligned && cells >= strips_from && trail_tile_supported(p, kNumTiles)) return kNumTiles;
+    return cells < 2000000 || (gauss && p.R == 1) ? 4 : 5;
+}
 bool trail_tile_supported(const DevParams& p, int tile) {
     if (tile == kTrailTileTma) return trail_tma_supported(p);
     if (tile < 0 || tile >= kNumTiles + kNumStream) return false;
@@ -209,36 +113,29 @@ bool trail_tile_streams(const DevParams& p, int tile) { return tile >= kNumTiles
 cudaError_t launch_trail_marks(const DevParams& p, int tile, const float* in, const uint8_t* marks_in, float* out,
                                uint8_t* marks_zero, cudaStream_t s, const cudaAccessPolicyWindow* win, bool pdl,
                                const TrailMaps* maps, int cur) {
-    if (!trail_tile_streams(p, tile)) return cudaErrorInvalidValue;
-    if (tile == kTrailTileTma) {
-        // without tensor maps, the 8-row streaming tile (same requirements, same bits)
-        if (!maps || !maps->ok) return launch_stream_rows<8>(p, in, marks_in, out, marks_zero, s, win, pdl);
-        return launch_trail_tma_marks(p, *maps, cur, in, marks_in, out, marks_zero, s, win, pdl);
-    }
+    if (!trail_tile_supported(p, tile)) tile = trail_tile_default(p, true);
+    // without tensor maps, the 8-row streaming tile (same requirements, same bits)
+    if (tile == kTrailTileTma && !(maps && maps->ok)) tile = kNumTiles;
     switch (tile) {
     case 7: return launch_stream_rows<8>(p, in, marks_in, out, marks_zero, s, win, pdl);
     case 8: return launch_stream_rows<16>(p, in, marks_in, out, marks_zero, s, win, pdl);
-    default: return launch_stream_rows<32>(p, in, marks_in, out, marks_zero, s, win, pdl);
+    case 9: return launch_stream_rows<32>(p, in, marks_in, out, marks_zero, s, win, pdl);
+    case kTrailTileTma: return launch_trail_tma_marks(p, *maps, cur, in, marks_in, out, marks_zero, s, win, pdl);
+    default: return launch_tile_index(tile, p, in, nullptr, marks_in, TileOut{out, nullptr, marks_zero}, s, win);
     }
 }
 
 cudaError_t launch_trail(const DevParams& p, int tile, const float* in, const uint32_t* counts_in, float* out,
                          uint32_t* counts_zero, cudaStream_t s, const cudaAccessPolicyWindow* win, bool pdl,
                          const TrailMaps* maps, int cur) {
-    if (!trail_tile_supported(p, tile) || (tile == kTrailTileTma && !(maps && maps->ok))) tile = trail_tile_default();
-    if (tile == kTrailTileTma) return launch_trail_tma(p, *maps, cur, in, counts_in, out, counts_zero, s, win, pdl);
+    if (!trail_tile_supported(p, tile)) tile = trail_tile_default(p, false);
+    if (tile == kTrailTileTma && !(maps && maps->ok)) tile = kNumTiles;
     switch (tile) {
-    case 0: return launch_tile<32, 8>(p, in, counts_in, out, counts_zero, s, win);
-    case 1: return launch_tile<64, 8>(p, in, counts_in, out, counts_zero, s, win);
-    case 2: return launch_tile<32, 16>(p, in, counts_in, out, counts_zero, s, win);
-    case 3: return launch_tile<64, 16>(p, in, counts_in, out, counts_zero, s, win);
-    case 4: return launch_tile<128, 8>(p, in, counts_in, out, counts_zero, s, win);
-    case 5: return launch_tile<128, 16>(p, in, counts_in, out, counts_zero, s, win);
-    case 6: return launch_tile<256, 8>(p, in, counts_in, out, counts_zero, s, win);
     case 7: return launch_stream_rows<8>(p, in, counts_in, out, counts_zero, s, win, pdl);
     case 8: return launch_stream_rows<16>(p, in, counts_in, out, counts_zero, s, win, pdl);
     case 9: return launch_stream_rows<32>(p, in, counts_in, out, counts_zero, s, win, pdl);
-    default: return cudaErrorInvalidValue;
+    case kTrailTileTma: return launch_trail_tma(p, *maps, cur, in, counts_in, out, counts_zero, s, win, pdl);
+    default: return launch_tile_index(tile, p, in, counts_in, nullptr, TileOut{out, counts_zero, nullptr}, s, win);
     }
 }
 

@@ -238,23 +238,23 @@ __device__ __forceinline__ void process_strip_m(const DevParams& p, const float*
         float o[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            float center = win[R].v[R + j];
-            float blur;
             if (kGauss) {
                 float acc = 0.0f;
 #pragma unroll
                 for (int q = 0; q <= 2 * R; q++) acc = slm_fma(p.w[q], hwin[q][j], acc);
-                blur = acc;
+                o[j] = acc;
             } else {
                 float sum = 0.0f;
 #pragma unroll
                 for (int dy = 0; dy < 3; dy++)
 #pragma unroll
                     for (int dx = 0; dx < 3; dx++) sum = slm_add(sum, win[dy].v[j + dx]);
-                blur = slm_div(sum, 9.0f);
+                o[j] = sum;
             }
-            o[j] = slm_mix(center, blur, p.rate);
         }
+        if (!kGauss) slm_div9x4(o);
+#pragma unroll
+        for (int j = 0; j < 4; j++) o[j] = slm_mix(win[R].v[R + j], o[j], p.rate);
         const size_t off = (size_t)y * W + c0;
         *reinterpret_cast<float4*>(out + off) = make_float4(o[0], o[1], o[2], o[3]);
         if (czero) zero_dep4(czero + off);

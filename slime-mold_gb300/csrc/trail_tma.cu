@@ -245,23 +245,23 @@ __global__ void __launch_bounds__(kTmaThreads) trail_tma_kernel(const __grid_con
         float res[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const float center = ctr[R][j];
-            float blur;
             if (kGauss) {
                 float acc = 0.0f;
 #pragma unroll
                 for (int q = 0; q <= 2 * R; q++) acc = slm_fma(p.w[q], hwin[q][j], acc);
-                blur = acc;
+                res[j] = acc;
             } else {
                 float sum = 0.0f;
 #pragma unroll
                 for (int dy = 0; dy < 3; dy++)
 #pragma unroll
                     for (int dx = 0; dx < 3; dx++) sum = slm_add(sum, win[dy][j + dx]);
-                blur = slm_div(sum, 9.0f);
+                res[j] = sum;
             }
-            res[j] = slm_mix(center, blur, p.rate);
         }
+        if (!kGauss) slm_div9x4(res);
+#pragma unroll
+        for (int j = 0; j < 4; j++) res[j] = slm_mix(ctr[R][j], res[j], p.rate);
         const size_t off = (size_t)y * W + x;
         *reinterpret_cast<float4*>(out + off) = make_float4(res[0], res[1], res[2], res[3]);
         if (dzero) zero_dep4(dzero + off);

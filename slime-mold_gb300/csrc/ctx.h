@@ -24,6 +24,15 @@ struct slime_ctx {
     uint64_t reorders_done = 0;
     slime::ReorderScratch reorder;
 
+    // A run of steps on a sorted copy of the agents (capi.cu): the copy's block
+    // (x | y | angle | speed | id, n_pad each), and the context's own agents
+    // while `agents` is the copy.
+    void* sorted_block = nullptr;
+    bool sorted_refused = false; // it did not fit: not tried again for these agents
+    bool in_sorted_run = false;
+    uint64_t sorted_since = 0; // steps_done at its last sort
+    slime::AgentsSoA own_agents;
+
     float* trail[2] = {nullptr, nullptr};
     cudaTextureObject_t trail_tex[2] = {0, 0}; // gather textures over trail[] (0 = none)
     slime::TrailMaps tmaps;                    // tensor maps over trail[], counts[], marks[] (tmaps.ok)
@@ -59,7 +68,7 @@ struct slime_ctx {
     // agent pass, bit 1 the trail pass; the autotuner may keep only one)
     unsigned l2_window_passes = 3;
 
-    std::map<std::pair<uint32_t, int>, cudaGraphExec_t> graphs; // (steps, start parity) -> graph
+    std::map<std::pair<uint32_t, int>, cudaGraphExec_t> graphs; // (steps, start parity | record << 1 | sorted copy << 2) -> graph
 
     uint64_t steps_done = 0;
     uint64_t launches = 0;
@@ -132,6 +141,13 @@ uint64_t kernels_per_step(const slime_ctx* ctx, bool marks);
 // the agents it updates first.
 int ensure_dispatch_order(slime_ctx* ctx);
 int run_steps(slime_ctx* ctx, uint32_t n);
+int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps);
+int resort_run(slime_ctx* ctx);
+int end_sorted_run(slime_ctx* ctx);
+void release_sorted(slime_ctx* ctx);
+cudaError_t ctx_alloc(slime_ctx* ctx, void** p, size_t bytes);
+// Steps after which a sorted copy is sorted again.
+uint32_t sorted_steps(const slime_ctx* ctx);
 int prepare_steps(slime_ctx* ctx, uint32_t n);
 void free_adjoint(slime_ctx* ctx);
 void setup_l2(slime_ctx* ctx);

@@ -572,8 +572,8 @@ int reorder_all(slime_ensemble* e) {
             const Colony& c = e->colonies[j];
             AgentsSoA a = colony_soa(e, c);
             ReorderScratch& scratch = l == 0 ? e->reorder : e->lane_reorder[l - 1];
-            ECK(launch_reorder(a, c.W, c.H, e->reorder_cell_log2, scratch, e->lanes[l]), "reordering agents");
-            e->launches += 5;
+            ECK(launch_reorder(a, a, c.W, c.H, e->reorder_cell_log2, scratch, e->lanes[l]), "reordering agents");
+            e->launches += kReorderKernels;
         }
         for (size_t l = 0; l < nr; l++) {
             ECK(cudaEventRecord(e->lane_ev[l], e->lanes[l]), "joining reorders");
@@ -583,8 +583,8 @@ int reorder_all(slime_ensemble* e) {
         for (const Colony& c : e->colonies) {
             if (c.n == 0) continue;
             AgentsSoA a = colony_soa(e, c);
-            ECK(launch_reorder(a, c.W, c.H, e->reorder_cell_log2, e->reorder, e->stream), "reordering agents");
-            e->launches += 5;
+            ECK(launch_reorder(a, a, c.W, c.H, e->reorder_cell_log2, e->reorder, e->stream), "reordering agents");
+            e->launches += kReorderKernels;
         }
     }
     e->last_reorder_step = e->steps_done;

@@ -32,6 +32,8 @@ struct AgentShape {
 int agent_shape_count();
 AgentShape agent_shape(int index);
 bool agent_shape_uses_texture(int index);
+// The shape of a context that neither chose nor tuned one.
+int agent_shape_default(uint64_t n, bool tex);
 // One agent pass (compute.wgsl:57-145): reads trail, adds deposit counts.
 // `tex` is a texture over `trail` (make_trail_texture) for the shapes that
 // sample through it; 0 runs those shapes on the pointer path.  With `marks`
@@ -132,16 +134,18 @@ cudaError_t launch_adjoint_step(const DevParams& p, const float* trail_s, const 
                                 cudaStream_t s);
 
 // ---- reorder.cu
-// Morton reordering of agent slots by cell; permutes SoA in place through
-// scratch buffers and keeps ids.
+// Morton reordering of agent slots by cell through scratch buffers; keeps ids.
 struct ReorderScratch {
     void* buf = nullptr;
     size_t bytes = 0;
 };
 cudaError_t launch_iota(uint32_t* ids, uint64_t n, cudaStream_t s);
-// Morton order; agents with id >= `visited` go to the last slots.
-cudaError_t launch_reorder(AgentsSoA& a, uint32_t W, uint32_t H, int cell_log2, ReorderScratch& scratch,
-                           cudaStream_t s, uint64_t visited = ~0ull);
+// The agents of `a` into `to` in Morton order (`to` may be `a` itself, with an id
+// array; without ids a's slots are the ids); agents with id >= `visited` go to
+// the last slots.  Six kernels.
+constexpr int kReorderKernels = 6;
+cudaError_t launch_reorder(const AgentsSoA& a, const AgentsSoA& to, uint32_t W, uint32_t H, int cell_log2,
+                           ReorderScratch& scratch, cudaStream_t s, uint64_t visited = ~0ull);
 
 // ---- colorize.cu
 cudaError_t launch_colorize(const float* trail, uint32_t W, uint32_t H, const uint8_t* lut, uint32_t tw,

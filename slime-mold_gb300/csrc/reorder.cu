@@ -8,8 +8,12 @@
 // reorder is a pure performance transform.
 //
 // Counting sort on the Morton code of the agent's (cell >> cell_log2):
-// key + histogram, exclusive scan, scatter to scratch, copy back.  The order
-// inside one key is whatever the scatter atomics produce.  Agents whose id is
+// key + histogram, exclusive scan, scatter to scratch as one 16-byte record and
+// an id per agent (a slot's five fields scattered each on its own would cost
+// five memory sectors an agent when the agents come unsorted, 160 bytes against
+// 64), and a pass that unpacks the records into the fields' arrays: the
+// agents' own, or another set, which is then sorted while the first stays as
+// it is.  The order inside one key is whatever the scatter atomics produce.  Agents whose id is
 // at or above `visited` (those the reference's dispatch never updates) get
 // one key past every Morton code, so they end up in the last slots and the
 // updated agents fill the first ones.
@@ -43,7 +47,7 @@ __global__ void key_hist_kernel(const float* __restrict__ x, const float* __rest
     int cx = min(max(slm_f2i(x[i]), 0), W - 1) >> cl;
     int cy = min(max(slm_f2i(y[i]), 0), H - 1) >> cl;
     uint32_t k = spread_bits((uint32_t)cx) | (spread_bits((uint32_t)cy) << 1);
-    if (visited < n && ids[i] >= visited) k = frozen_key;
+    if (visited < n && (ids ? ids[i] : (uint32_t)i) >= visited) k = frozen_key;
     keys[i] = k;
     const unsigned group = __match_any_sync(__activemask(), k);
     if ((int)(threadIdx.x & 31) == __ffs(group) - 1) atomicAdd(hist + k, (uint32_t)__popc(group));
@@ -127,11 +131,12 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(uint32_t* __re
 __global__ void scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
                                const float* __restrict__ th, const float* __restrict__ v,
                                const uint32_t* __restrict__ ids, const uint32_t* __restrict__ keys, uint64_t n,
-                               uint32_t* __restrict__ offsets, float* __restrict__ tx, float* __restrict__ ty,
-                               float* __restrict__ tth, float* __restrict__ tv, uint32_t* __restrict__ tid) {
+                               uint32_t* __restrict__ offsets, float4* __restrict__ rec, uint32_t* __restrict__ rid) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t k = keys[i];
+    const float4 a = make_float4(__ldcs(x + i), __ldcs(y + i), __ldcs(th + i), __ldcs(v + i));
+    const uint32_t id = ids ? __ldcs(ids + i) : (uint32_t)i;
     const unsigned active = __activemask();
     const unsigned group = __match_any_sync(active, k);
     const int lane = (int)(threadIdx.x & 31);
@@ -141,11 +146,21 @@ __global__ void scatter_kernel(const float* __restrict__ x, const float* __restr
     base = __shfl_sync(active, base, leader);
     // slots of one key are claimed in lane order within the warp
     const uint32_t pos = base + (uint32_t)__popc(group & ((1u << lane) - 1u));
-    tx[pos] = x[i];
-    ty[pos] = y[i];
-    tth[pos] = th[i];
-    tv[pos] = v[i];
-    tid[pos] = ids[i];
+    rec[pos] = a;
+    rid[pos] = id;
+}
+
+__global__ void unpack_kernel(const float4* __restrict__ rec, const uint32_t* __restrict__ rid, uint64_t n,
+                              float* __restrict__ x, float* __restrict__ y, float* __restrict__ th,
+                              float* __restrict__ v, uint32_t* __restrict__ ids) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 a = __ldcs(rec + i);
+    x[i] = a.x;
+    y[i] = a.y;
+    th[i] = a.z;
+    v[i] = a.w;
+    ids[i] = __ldcs(rid + i);
 }
 
 __global__ void iota_kernel(uint32_t* __restrict__ ids, uint64_t n) {
@@ -163,10 +178,10 @@ cudaError_t launch_iota(uint32_t* ids, uint64_t n, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_reorder(AgentsSoA& a, uint32_t W, uint32_t H, int cell_log2, ReorderScratch& scratch,
-                           cudaStream_t s, uint64_t visited) {
+cudaError_t launch_reorder(const AgentsSoA& a, const AgentsSoA& to, uint32_t W, uint32_t H, int cell_log2,
+                           ReorderScratch& scratch, cudaStream_t s, uint64_t visited) {
     if (a.n == 0) return cudaSuccess;
-    if (!a.ids) return cudaErrorInvalidValue; // the caller installs identity ids first
+    if (!to.ids) return cudaErrorInvalidValue;
     if (cell_log2 < 0) cell_log2 = 0;
     if (cell_log2 > 15) cell_log2 = 15;
     uint32_t dx = (W + (1u << cell_log2) - 1) >> cell_log2;
@@ -182,7 +197,7 @@ cudaError_t launch_reorder(AgentsSoA& a, uint32_t W, uint32_t H, int cell_log2, 
     uint64_t nblk = (nb + kScanTile - 1) / kScanTile;
     const uint64_t n = a.n;
     size_t need = align256(4 * n) /*keys*/ + align256(4 * nb) /*hist*/ + align256(4 * nblk) /*block sums*/ +
-                  4 * align256(4 * n) /*x y th v*/ + align256(4 * n) /*ids*/;
+                  align256(16 * n) /*records*/ + align256(4 * n) /*ids*/;
     if (scratch.bytes < need) {
         if (scratch.buf) dev_free(scratch.buf);
         scratch.buf = nullptr;
@@ -195,11 +210,8 @@ cudaError_t launch_reorder(AgentsSoA& a, uint32_t W, uint32_t H, int cell_log2, 
     uint32_t* keys = (uint32_t*)p; p += align256(4 * n);
     uint32_t* hist = (uint32_t*)p; p += align256(4 * nb);
     uint32_t* bsum = (uint32_t*)p; p += align256(4 * nblk);
-    float* tx = (float*)p; p += align256(4 * n);
-    float* ty = (float*)p; p += align256(4 * n);
-    float* tth = (float*)p; p += align256(4 * n);
-    float* tv = (float*)p; p += align256(4 * n);
-    uint32_t* tid = (uint32_t*)p;
+    float4* rec = (float4*)p; p += align256(16 * n);
+    uint32_t* rid = (uint32_t*)p;
 
     cudaError_t e = cudaMemsetAsync(hist, 0, 4 * nb, s);
     if (e != cudaSuccess) return e;
@@ -209,13 +221,9 @@ cudaError_t launch_reorder(AgentsSoA& a, uint32_t W, uint32_t H, int cell_log2, 
     scan_reduce_kernel<<<(unsigned)nblk, kScanThreads, 0, s>>>(hist, nb, bsum);
     scan_block_sums_kernel<<<1, kScanThreads, 0, s>>>(bsum, (uint32_t)nblk);
     scan_apply_kernel<<<(unsigned)nblk, kScanThreads, 0, s>>>(hist, nb, bsum);
-    scatter_kernel<<<blocks, 256, 0, s>>>(a.x, a.y, a.th, a.v, a.ids, keys, n, hist, tx, ty, tth, tv, tid);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(a.x, tx, 4 * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(a.y, ty, 4 * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(a.th, tth, 4 * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(a.v, tv, 4 * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
-    return cudaMemcpyAsync(a.ids, tid, 4 * n, cudaMemcpyDeviceToDevice, s);
+    scatter_kernel<<<blocks, 256, 0, s>>>(a.x, a.y, a.th, a.v, a.ids, keys, n, hist, rec, rid);
+    unpack_kernel<<<blocks, 256, 0, s>>>(rec, rid, n, to.x, to.y, to.th, to.v, to.ids);
+    return cudaGetLastError();
 }
 
 } // namespace slime

@@ -16,164 +16,407 @@
 // the backward replays each segment from its checkpoint (bit-identical to the
 // recorded run), keeps T_s and k_s of the segment in HBM, and runs one fused
 // stencil kernel per step backwards through it.
+#include <string.h>
+
 #include "ctx.h"
+#include "trail_tile.cuh"
 
 using namespace slime;
 
 namespace slime {
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kTW = 64, kTH = 16;
+// One backward step.  A block takes a tile of 128 x 16 cells, a thread four
+// adjacent columns of every fourth row, and stages the window of u (T_s folded
+// and decayed) and of g with 16-byte loads.  What bounded it before were the
+// block's sums (three binary64 butterflies over all its threads, on a GPU with
+// two binary64 operations per SM and cycle), a second read of T and k for the
+// thread's own cells, and one cell per thread per pass through shared memory:
+//   * a thread sums each of its columns' four cells in binary32, and keeps its
+//     three sums over all steps as unevaluated binary32 pairs in memory
+//     (T. Dekker, "A floating-point technique for extending the available
+//     precision", Numer. Math. 18, 1971: what an addition rounds off goes into
+//     the second number); they are added up in binary64 once per backward, in
+//     one order, so the gradients do not depend on which block finishes first;
+//   * a thread's own cells of T and k are read once (with a shared-memory
+//     carve-out this large nothing stays in L1 for a second read), folded once
+//     and kept in registers, as is its g;
+//   * u is staged before the wait for the step it follows, which writes only g.
+// The blur of g is separable; B(u) - u, small against u, is summed term by term
+// from neighbour-minus-centre differences.  Sum by sum the arithmetic of the
+// kernel before: 1024^2, radius 1, 22.6 us a step then, 8.7 now (16.8 MB
+// of T, k and g: 2.5 us at the measured copy bandwidth).
+constexpr int kTW = 128, kTH = 16;
+constexpr int kSlots = 4;              // a thread's rows are its slot and every fourth after it
+constexpr int kRows = kTH / kSlots;
+constexpr int kThreads = kTW / 4 * kSlots;
 
-__device__ __forceinline__ double block_sum(double v, double* red) {
+// s.x + s.y += x: what the sum s.x + x rounds off (Knuth's two-sum) joins s.y.
+__device__ __forceinline__ void pair_add(float2& s, float x) {
+    const float t = slm_add(s.x, x);
+    const float b = slm_sub(t, s.x);
+    s.y = slm_add(s.y, slm_add(slm_sub(s.x, slm_sub(t, b)), slm_sub(x, b)));
+    s.x = t;
+}
+
+// The first n of four cells from i.
+__device__ __forceinline__ float4 row4(const float* __restrict__ a, size_t i, int n) {
+    return make_float4(n > 0 ? __ldg(a + i) : 0.0f, n > 1 ? __ldg(a + i + 1) : 0.0f, n > 2 ? __ldg(a + i + 2) : 0.0f,
+                       n > 3 ? __ldg(a + i + 3) : 0.0f);
+}
+__device__ __forceinline__ uint4 row4(const uint32_t* __restrict__ a, size_t i, int n) {
+    return make_uint4(n > 0 ? __ldg(a + i) : 0u, n > 1 ? __ldg(a + i + 1) : 0u, n > 2 ? __ldg(a + i + 2) : 0u,
+                      n > 3 ? __ldg(a + i + 3) : 0u);
+}
+
+// Columns 4c - LP .. 4c + 3 + LP of a window row (row points at column 4c - LP).
+template <int LP>
+__device__ __forceinline__ void window4(const float* row, float* e) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < kThreads / 32; w++) t += red[w];
-    __syncthreads();
-    return t;
+    for (int i = 0; i < 1 + LP / 2; i++) {
+        const float4 v = *reinterpret_cast<const float4*>(row + 4 * i);
+        e[4 * i] = v.x, e[4 * i + 1] = v.y, e[4 * i + 2] = v.z, e[4 * i + 3] = v.w;
+    }
+}
+
+// The 2R halo rows of a window, spread over the slots: window row of a slot's
+// i-th one, or -1.
+template <int R>
+__device__ __forceinline__ int halo_row(int slot, int i) {
+    const int h = slot + i * kSlots;
+    return h >= 2 * R ? -1 : (h < R ? h : kTH + h);
+}
+
+__device__ __forceinline__ float4 decayed(const DevParams& p, const float4& f) {
+    return make_float4(apply_decay(p, f.x), apply_decay(p, f.y), apply_decay(p, f.z), apply_decay(p, f.w));
+}
+__device__ __forceinline__ float4 folded(const DevParams& p, const float4& t, const uint4& k) {
+    return make_float4(fold_deposits(t.x, k.x, p.dep), fold_deposits(t.y, k.y, p.dep), fold_deposits(t.z, k.z, p.dep),
+                       fold_deposits(t.w, k.w, p.dep));
 }
 
 template <int R, bool kGauss>
 __global__ void __launch_bounds__(kThreads) adjoint_kernel(const __grid_constant__ DevParams p,
-                                                           const float* __restrict__ T,
-                                                           const uint32_t* __restrict__ K,
-                                                           const float* __restrict__ gin, float* __restrict__ gout,
-                                                           double* __restrict__ acc, uint32_t rate_active) {
-    constexpr int SW = kTW + 2 * R, SH = kTH + 2 * R;
-    extern __shared__ float sm[];
+                                                           const float* __restrict__ T, const uint32_t* __restrict__ K,
+                                                           const float* gin, float* gout, float2* acc,
+                                                           uint32_t rate_active, int tiles_x, int vec) {
+    typedef TileGeom<kTW, kTH, R> G; // window layout
+    constexpr int NH = (2 * R + kSlots - 1) / kSlots; // halo rows per slot
+    extern __shared__ __align__(16) float sm[];
     float* su = sm;
-    float* sg = sm + SH * SW;
-    float* hg = sg + SH * SW; // Gaussian only: horizontal pass of g
-    __shared__ double red[kThreads / 32];
+    float* sg = sm + G::window;
+    float* hg = sg + G::window; // Gaussian only: the rows of g blurred
     const int W = p.W, H = p.H;
-    const int x0 = blockIdx.x * kTW, y0 = blockIdx.y * kTH;
-    for (int i = threadIdx.x; i < SH * SW; i += kThreads) {
-        int ly = i / SW, lx = i - ly * SW;
-        int gi = wrap_coord(y0 + ly - R, H) * W + wrap_coord(x0 + lx - R, W);
-        su[i] = apply_decay(p, fold_deposits(__ldg(T + gi), __ldg(K + gi), p.dep));
-        sg[i] = __ldg(gin + gi);
-    }
-    __syncthreads();
-    if (kGauss) {
-        for (int i = threadIdx.x; i < SH * kTW; i += kThreads) {
-            int ly = i / kTW, lx = i - ly * kTW;
-            float b = 0.0f;
+    const int by = blockIdx.x / tiles_x;
+    const int x0 = (blockIdx.x - by * tiles_x) * kTW, y0 = by * kTH;
+    const int c = threadIdx.x & 31, slot = threadIdx.x >> 5;
+    const int gx = wrap_coord(x0 + 4 * c, W);
+    constexpr int NC = (kTW + 2 * R + 31) / 32; // rows of any width: cells per lane and row, and their columns
+    int cols[NC];
 #pragma unroll
-            for (int t = 0; t <= 2 * R; t++) b = slm_fma(p.w[t], sg[ly * SW + lx + t], b);
-            hg[i] = b;
+    for (int q = 0; q < NC; q++) cols[q] = wrap_coord(x0 - R + min(c + 32 * q, kTW + 2 * R - 1), W);
+    float4 f4[kRows], g4[kRows];
+    uint4 k4[kRows];
+    constexpr int HN = G::SH * 2 * R; // halo columns: 2R cells of every window row
+    if (vec) {
+        float4 th[NH > 0 ? NH : 1];
+        uint4 kh[NH > 0 ? NH : 1];
+#pragma unroll
+        for (int i = 0; i < kRows; i++) {
+            const size_t at = (size_t)wrap_coord(y0 + slot + i * kSlots, H) * W + gx;
+            f4[i] = __ldg(reinterpret_cast<const float4*>(T + at));
+            k4[i] = __ldg(reinterpret_cast<const uint4*>(K + at));
+        }
+#pragma unroll
+        for (int i = 0; i < NH; i++) {
+            const int r = halo_row<R>(slot, i);
+            if (r >= 0) {
+                const size_t at = (size_t)wrap_coord(y0 - R + r, H) * W + gx;
+                th[i] = __ldg(reinterpret_cast<const float4*>(T + at));
+                kh[i] = __ldg(reinterpret_cast<const uint4*>(K + at));
+            }
+        }
+        for (int i = threadIdx.x; i < HN; i += kThreads) {
+            const int r = i / (2 * R > 0 ? 2 * R : 1), j = i - r * 2 * R;
+            const int cc = j < R ? j - R : kTW + j - R;
+            const size_t at = (size_t)wrap_coord(y0 - R + r, H) * W + wrap_coord(x0 + cc, W);
+            su[r * G::stride + G::LP + cc] = apply_decay(p, fold_deposits(__ldg(T + at), __ldg(K + at), p.dep));
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; i++) {
+            f4[i] = folded(p, f4[i], k4[i]);
+            *reinterpret_cast<float4*>(su + (R + slot + i * kSlots) * G::stride + G::LP + 4 * c) = decayed(p, f4[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < NH; i++) {
+            const int r = halo_row<R>(slot, i);
+            if (r >= 0)
+                *reinterpret_cast<float4*>(su + r * G::stride + G::LP + 4 * c) = decayed(p, folded(p, th[i], kh[i]));
+        }
+    } else {
+#pragma unroll 2
+        for (int r = slot; r < G::SH; r += kSlots) {
+            const size_t row = (size_t)wrap_coord(y0 - R + r, H) * W;
+            float t[NC];
+            uint32_t k[NC];
+#pragma unroll
+            for (int q = 0; q < NC; q++) {
+                t[q] = __ldg(T + row + cols[q]);
+                k[q] = __ldg(K + row + cols[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < NC; q++)
+                if (c + 32 * q < kTW + 2 * R)
+                    su[r * G::stride + G::LP - R + c + 32 * q] = apply_decay(p, fold_deposits(t[q], k[q], p.dep));
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; i++) {
+            const int gy = y0 + slot + i * kSlots, n = gy < H ? min(4, W - (x0 + 4 * c)) : 0;
+            const size_t at = (size_t)gy * W + x0 + 4 * c;
+            k4[i] = row4(K, at, n);
+            f4[i] = folded(p, row4(T, at, n), k4[i]);
+        }
+    }
+    // g and the sums are the output of the step this one follows
+    pdl_wait();
+    pdl_trigger();
+    float2* own_acc = acc + (size_t)blockIdx.x * (3 * kThreads) + threadIdx.x;
+    float2 s[3] = {own_acc[0], own_acc[kThreads], own_acc[2 * kThreads]};
+    if (vec) {
+        float4 gh[NH > 0 ? NH : 1];
+#pragma unroll
+        for (int i = 0; i < kRows; i++)
+            g4[i] = *reinterpret_cast<const float4*>(gin + (size_t)wrap_coord(y0 + slot + i * kSlots, H) * W + gx);
+#pragma unroll
+        for (int i = 0; i < NH; i++) {
+            const int r = halo_row<R>(slot, i);
+            if (r >= 0) gh[i] = *reinterpret_cast<const float4*>(gin + (size_t)wrap_coord(y0 - R + r, H) * W + gx);
+        }
+        for (int i = threadIdx.x; i < HN; i += kThreads) {
+            const int r = i / (2 * R > 0 ? 2 * R : 1), j = i - r * 2 * R;
+            const int cc = j < R ? j - R : kTW + j - R;
+            sg[r * G::stride + G::LP + cc] = gin[(size_t)wrap_coord(y0 - R + r, H) * W + wrap_coord(x0 + cc, W)];
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; i++)
+            *reinterpret_cast<float4*>(sg + (R + slot + i * kSlots) * G::stride + G::LP + 4 * c) = g4[i];
+#pragma unroll
+        for (int i = 0; i < NH; i++) {
+            const int r = halo_row<R>(slot, i);
+            if (r >= 0) *reinterpret_cast<float4*>(sg + r * G::stride + G::LP + 4 * c) = gh[i];
+        }
+        __syncthreads();
+    } else {
+#pragma unroll 2
+        for (int r = slot; r < G::SH; r += kSlots) {
+            const size_t row = (size_t)wrap_coord(y0 - R + r, H) * W;
+            float t[NC];
+#pragma unroll
+            for (int q = 0; q < NC; q++) t[q] = gin[row + cols[q]];
+#pragma unroll
+            for (int q = 0; q < NC; q++)
+                if (c + 32 * q < kTW + 2 * R) sg[r * G::stride + G::LP - R + c + 32 * q] = t[q];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kRows; i++)
+            g4[i] = *reinterpret_cast<const float4*>(sg + (R + slot + i * kSlots) * G::stride + G::LP + 4 * c);
+    }
+    if (kGauss) {
+        for (int r = slot; r < G::SH; r += kSlots) {
+            float e[4 + 2 * G::LP], b[4];
+            window4<G::LP>(sg + r * G::stride + 4 * c, e);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                b[j] = 0.0f;
+#pragma unroll
+                for (int t = 0; t <= 2 * R; t++) b[j] = slm_fma(p.w[t], e[G::LP - R + j + t], b[j]);
+            }
+            *reinterpret_cast<float4*>(hg + r * kTW + 4 * c) = make_float4(b[0], b[1], b[2], b[3]);
         }
         __syncthreads();
     }
-    float sd = 0.0f, sr = 0.0f, sp = 0.0f;
     const float r = p.rate;
-    for (int i = threadIdx.x; i < kTW * kTH; i += kThreads) {
-        int ly = i / kTW, lx = i - ly * kTW;
-        int gx = x0 + lx, gy = y0 + ly;
-        if (gx >= W || gy >= H) continue;
-        int c = (ly + R) * SW + lx + R;
-        float u = su[c], g = sg[c];
-        // B(g) for the adjoint of the blur, and B(u) - u for the rate
-        // gradient in difference form (B(u) - u is small against u, so it is
-        // summed from neighbour-minus-centre differences).
-        float bg, bmu;
+    float sd[4] = {}, sr[4] = {}, sp[4] = {}; // by column
+#pragma unroll
+    for (int i = 0; i < kRows; i++) {
+        const int ry = slot + i * kSlots; // row of the tile
+        const int gy = y0 + ry;
+        const int n = gy < H ? min(4, W - (x0 + 4 * c)) : 0; // cells of this thread in the row
+        if (n <= 0) continue;
+        float bg[4], bmu[4]; // B(g), B(u) - u
+        const float4 uc4 = *reinterpret_cast<const float4*>(su + (R + ry) * G::stride + G::LP + 4 * c);
+        const float uc[4] = {uc4.x, uc4.y, uc4.z, uc4.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) bg[j] = bmu[j] = 0.0f;
         if (kGauss) {
-            float b = 0.0f;
 #pragma unroll
-            for (int t = 0; t <= 2 * R; t++) b = slm_fma(p.w[t], hg[(ly + t) * kTW + lx], b);
-            bg = b;
-            float dsum = 0.0f;
-#pragma unroll
-            for (int dy = 0; dy <= 2 * R; dy++) {
-                float row = 0.0f;
-#pragma unroll
-                for (int dx = 0; dx <= 2 * R; dx++) row += p.w[dx] * (su[(ly + dy) * SW + lx + dx] - u);
-                dsum += p.w[dy] * row;
+            for (int t = 0; t <= 2 * R; t++) {
+                const float4 a = *reinterpret_cast<const float4*>(hg + (ry + t) * kTW + 4 * c);
+                bg[0] = slm_fma(p.w[t], a.x, bg[0]);
+                bg[1] = slm_fma(p.w[t], a.y, bg[1]);
+                bg[2] = slm_fma(p.w[t], a.z, bg[2]);
+                bg[3] = slm_fma(p.w[t], a.w, bg[3]);
             }
-            bmu = dsum + p.w2sum_m1 * u;
-        } else {
-            float b = 0.0f, dsum = 0.0f;
+            if (rate_active) {
+                for (int t = 0; t <= 2 * R; t++) {
+                    float e[4 + 2 * G::LP];
+                    window4<G::LP>(su + (ry + t) * G::stride + 4 * c, e);
 #pragma unroll
-            for (int dy = -1; dy <= 1; dy++)
+                    for (int j = 0; j < 4; j++) {
+                        float row = 0.0f;
 #pragma unroll
-                for (int dx = -1; dx <= 1; dx++) {
-                    b += sg[c + dy * SW + dx];
-                    dsum += su[c + dy * SW + dx] - u;
+                        for (int d = 0; d <= 2 * R; d++) row += p.w[d] * (e[G::LP - R + j + d] - uc[j]);
+                        bmu[j] += p.w[t] * row;
+                    }
                 }
-            bg = b * (1.0f / 9.0f);
-            bmu = dsum * (1.0f / 9.0f);
-        }
-        if (rate_active) sr += g * bmu;
-        float g_u = (1.0f - r) * g + r * bg;
-        int gi = gy * W + gx;
-        uint32_t k = __ldg(K + gi);
-        float f = fold_deposits(__ldg(T + gi), k, p.dep);
-        float g_f;
-        if (p.decay_mode == SLIME_DECAY_MULTIPLY) {
-            sd += g_u * f;
-            g_f = p.decay * g_u;
+#pragma unroll
+                for (int j = 0; j < 4; j++) bmu[j] = bmu[j] + p.w2sum_m1 * uc[j];
+            }
         } else {
-            bool act = slm_sub(f, p.decay_k) > 0.0f;
-            sd += act ? -0.001f * g_u : 0.0f;
-            g_f = act ? g_u : 0.0f;
+#pragma unroll
+            for (int dy = 0; dy < 3; dy++) {
+                const float* rg = sg + (ry + dy) * G::stride + G::LP + 4 * c;
+                const float* ru = su + (ry + dy) * G::stride + G::LP + 4 * c;
+                const float4 vg = *reinterpret_cast<const float4*>(rg), vu = *reinterpret_cast<const float4*>(ru);
+                const float eg[6] = {rg[-1], vg.x, vg.y, vg.z, vg.w, rg[4]};
+                const float eu[6] = {ru[-1], vu.x, vu.y, vu.z, vu.w, ru[4]};
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int dx = 0; dx < 3; dx++) {
+                        bg[j] += eg[j + dx];
+                        bmu[j] += eu[j + dx] - uc[j];
+                    }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                bg[j] = bg[j] * (1.0f / 9.0f);
+                bmu[j] = bmu[j] * (1.0f / 9.0f);
+            }
         }
-        bool unclamped = (k == 0u) || (f > 0.0f && f < 1.0f);
-        if (unclamped) sp += g_f * (float)k;
-        gout[gi] = unclamped ? g_f : 0.0f;
+        const float fv[4] = {f4[i].x, f4[i].y, f4[i].z, f4[i].w}, gv[4] = {g4[i].x, g4[i].y, g4[i].z, g4[i].w};
+        const uint32_t kv[4] = {k4[i].x, k4[i].y, k4[i].z, k4[i].w};
+        float o[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float g = gv[j], f = fv[j];
+            const uint32_t k = kv[j];
+            const float g_u = (1.0f - r) * g + r * bg[j];
+            float g_f, d_decay;
+            if (p.decay_mode == SLIME_DECAY_MULTIPLY) {
+                d_decay = g_u * f;
+                g_f = p.decay * g_u;
+            } else {
+                const bool act = slm_sub(f, p.decay_k) > 0.0f;
+                d_decay = act ? -0.001f * g_u : 0.0f;
+                g_f = act ? g_u : 0.0f;
+            }
+            const bool unclamped = (k == 0u) || (f > 0.0f && f < 1.0f);
+            if (j < n) {
+                sd[j] += d_decay;
+                if (rate_active) sr[j] += g * bmu[j];
+                if (unclamped) sp[j] += g_f * (float)k;
+            }
+            o[j] = unclamped ? g_f : 0.0f;
+        }
+        const size_t at = (size_t)gy * W + x0 + 4 * c;
+        if (vec) {
+            *reinterpret_cast<float4*>(gout + at) = make_float4(o[0], o[1], o[2], o[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (j < n) gout[at + j] = o[j];
+        }
     }
-    double td = block_sum((double)sd, red);
-    double tr = block_sum((double)sr, red);
-    double tp = block_sum((double)sp, red);
-    if (threadIdx.x == 0) {
-        atomicAdd(acc + 0, td);
-        atomicAdd(acc + 1, tr);
-        atomicAdd(acc + 2, tp);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        pair_add(s[0], sd[j]);
+        pair_add(s[1], sr[j]);
+        pair_add(s[2], sp[j]);
     }
+    own_acc[0] = s[0];
+    own_acc[kThreads] = s[1];
+    own_acc[2 * kThreads] = s[2];
+}
+
+constexpr uint32_t kSumBlocks = kThreads; // blocks of the first pass over the threads' sums
+
+// The threads' sums, in two passes, each in a fixed order.
+__device__ __forceinline__ double block_sum(double v) {
+    __shared__ double s[kThreads];
+    s[threadIdx.x] = v;
+    __syncthreads();
+    for (int o = kThreads / 2; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
+        __syncthreads();
+    }
+    return s[0];
+}
+__global__ void __launch_bounds__(kThreads) sum_threads_kernel(const float2* __restrict__ acc, uint32_t blocks,
+                                                          double* __restrict__ part) {
+    double v = 0.0;
+    for (uint32_t b = blockIdx.x; b < blocks; b += kSumBlocks) {
+        const float2 a = acc[((size_t)b * 3 + blockIdx.y) * kThreads + threadIdx.x];
+        // an infinite or NaN sum says nothing in its second number
+        v += (double)a.x + (fabsf(a.x) <= 3.0e38f ? (double)a.y : 0.0);
+    }
+    v = block_sum(v);
+    if (threadIdx.x == 0) part[blockIdx.y * kSumBlocks + blockIdx.x] = v;
+}
+__global__ void __launch_bounds__(kThreads) sum_parts_kernel(const double* __restrict__ part, double* __restrict__ out) {
+    const double v = block_sum(part[blockIdx.x * kSumBlocks + threadIdx.x]);
+    if (threadIdx.x == 0) out[blockIdx.x] = v;
+}
+
+uint32_t adjoint_blocks(uint32_t W, uint32_t H) {
+    return ((W + kTW - 1) / kTW) * ((H + kTH - 1) / kTH);
 }
 
 template <int R, bool kGauss>
 cudaError_t launch_adj(const DevParams& p, const float* T, const uint32_t* K, const float* gin, float* gout,
-                       double* acc, uint32_t rate_active, cudaStream_t s) {
-    constexpr int SW = kTW + 2 * R, SH = kTH + 2 * R;
-    size_t smem = sizeof(float) * (2 * SH * SW + (kGauss ? SH * kTW : 0));
+                       float2* acc, uint32_t rate_active, cudaStream_t s, bool pdl) {
+    typedef TileGeom<kTW, kTH, R> G;
+    const size_t smem = sizeof(float) * (2 * G::window + (kGauss ? G::SH * kTW : 0));
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(adjoint_kernel<R, kGauss>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return e;
     }
-    dim3 grid((p.W + kTW - 1) / kTW, (p.H + kTH - 1) / kTH);
-    adjoint_kernel<R, kGauss><<<grid, kThreads, smem, s>>>(p, T, K, gin, gout, acc, rate_active);
-    return cudaGetLastError();
+    const int vec = p.W % 4 == 0 && (((uintptr_t)T | (uintptr_t)K | (uintptr_t)gin | (uintptr_t)gout) & 15) == 0;
+    return launch_kp(adjoint_kernel<R, kGauss>, dim3(adjoint_blocks((uint32_t)p.W, (uint32_t)p.H)), dim3(kThreads), smem, s,
+                     nullptr, pdl, p, T, K, gin, gout, acc, rate_active, (p.W + kTW - 1) / kTW, vec);
 }
 
 } // namespace
 
 cudaError_t launch_adjoint_step(const DevParams& p, const float* T, const uint32_t* K, const float* gin,
-                                float* gout, double* acc, uint32_t rate_active, cudaStream_t s) {
-    if (p.blur_mode != SLIME_BLUR_GAUSS) return launch_adj<1, false>(p, T, K, gin, gout, acc, rate_active, s);
+                                float* gout, float2* acc, uint32_t rate_active, cudaStream_t s, bool pdl) {
+    if (p.blur_mode != SLIME_BLUR_GAUSS) return launch_adj<1, false>(p, T, K, gin, gout, acc, rate_active, s, pdl);
     switch (p.R) {
-    case 0: return launch_adj<0, true>(p, T, K, gin, gout, acc, rate_active, s);
-    case 1: return launch_adj<1, true>(p, T, K, gin, gout, acc, rate_active, s);
-    case 2: return launch_adj<2, true>(p, T, K, gin, gout, acc, rate_active, s);
-    case 3: return launch_adj<3, true>(p, T, K, gin, gout, acc, rate_active, s);
-    case 4: return launch_adj<4, true>(p, T, K, gin, gout, acc, rate_active, s);
-    case 5: return launch_adj<5, true>(p, T, K, gin, gout, acc, rate_active, s);
-    case 6: return launch_adj<6, true>(p, T, K, gin, gout, acc, rate_active, s);
-    case 7: return launch_adj<7, true>(p, T, K, gin, gout, acc, rate_active, s);
-    case 8: return launch_adj<8, true>(p, T, K, gin, gout, acc, rate_active, s);
+    case 0: return launch_adj<0, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
+    case 1: return launch_adj<1, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
+    case 2: return launch_adj<2, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
+    case 3: return launch_adj<3, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
+    case 4: return launch_adj<4, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
+    case 5: return launch_adj<5, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
+    case 6: return launch_adj<6, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
+    case 7: return launch_adj<7, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
+    case 8: return launch_adj<8, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
     default: return cudaErrorInvalidValue;
     }
 }
 
+void drop_segment_graphs(slime_ctx* ctx) {
+    for (auto& kv : ctx->adj.seg_graphs) cudaGraphExecDestroy(kv.second);
+    ctx->adj.seg_graphs.clear();
+}
+
 void free_adjoint(slime_ctx* ctx) {
     auto& a = ctx->adj;
-    for (auto& kv : a.seg_graphs) cudaGraphExecDestroy(kv.second);
-    a.seg_graphs.clear();
+    drop_segment_graphs(ctx);
+    for (cudaTextureObject_t t : a.seg_tex)
+        if (t) cudaDestroyTextureObject(t);
     void* ptrs[] = {a.ckpt_agents, a.ckpt_ids, a.ckpt_trail, a.seg_trail, a.seg_counts, a.g[0], a.g[1],
                     a.acc, a.agents_tmp, a.ids_tmp};
     for (void* q : ptrs)
@@ -189,6 +432,75 @@ void free_adjoint(slime_ctx* ctx) {
         if (_e != cudaSuccess) return cuda_error(ctx->err, _e, what);                                       \
     } while (0)
 
+namespace {
+
+// Cells from one step's trail (or counts) of a segment to the next one's: rows
+// of every step 256-byte aligned, for 16-byte loads and gather textures.
+size_t segment_stride(const slime_ctx* ctx) { return ((size_t)ctx->W * ctx->H + 63) & ~(size_t)63; }
+
+// The recorded steps, on the context's agents as they are now (its own, or the
+// sorted copy of begin_sorted_run).
+int record_steps(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) {
+    auto& a = ctx->adj;
+    const size_t cells = (size_t)ctx->W * ctx->H;
+    const uint64_t n_pad = ctx->agents.n_pad;
+    const uint32_t K = ckpt_every < n_steps ? ckpt_every : n_steps;
+    const uint32_t n_ckpt = (n_steps + K - 1) / K;
+    const bool with_ids = ctx->agents.ids != nullptr;
+    // the last recording's buffers serve this one when it is of the same size
+    if (a.ckpt_trail && (a.n_ckpt != n_ckpt || a.ckpt_every != K || a.n != ctx->agents.n || a.n_pad != n_pad ||
+                         a.with_ids != with_ids))
+        free_adjoint(ctx);
+    if (memcmp(&a.dev, &ctx->dev, sizeof a.dev) != 0 || a.tile != ctx->tile || a.agent_shape != ctx->agent_shape)
+        drop_segment_graphs(ctx);
+    a.recorded = false;
+    a.n_steps = n_steps;
+    a.ckpt_every = K;
+    a.n_ckpt = n_ckpt;
+    a.dev = ctx->dev;
+    a.tile = ctx->tile;
+    a.agent_shape = ctx->agent_shape;
+    const uint32_t rate_active = (ctx->params.diffusion_rate > 0.0f && ctx->params.diffusion_rate < 1.0f) ? 1u : 0u;
+    if (rate_active != a.rate_active) drop_segment_graphs(ctx);
+    a.rate_active = rate_active;
+    a.n = ctx->agents.n;
+    a.n_pad = n_pad;
+    a.with_ids = with_ids;
+    cudaError_t e;
+    if (!a.ckpt_trail &&
+        ((e = ctx_alloc(ctx, (void**)&a.ckpt_agents, (size_t)a.n_ckpt * 4 * n_pad * sizeof(float))) != cudaSuccess ||
+         (a.with_ids && (e = ctx_alloc(ctx, (void**)&a.ckpt_ids, (size_t)a.n_ckpt * n_pad * sizeof(uint32_t))) != cudaSuccess) ||
+         (e = ctx_alloc(ctx, (void**)&a.ckpt_trail, (size_t)a.n_ckpt * cells * sizeof(float))) != cudaSuccess)) {
+        free_adjoint(ctx);
+        return cuda_error(ctx->err, e, "allocating checkpoints");
+    }
+    for (uint32_t j = 0; j < a.n_ckpt; j++) {
+        int rc = resort_run(ctx);
+        if (rc != SLIME_OK) return rc;
+        CK(cudaMemcpyAsync(a.ckpt_agents + (size_t)j * 4 * n_pad, ctx->agents.x, 4 * n_pad * sizeof(float),
+                           cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing agents");
+        if (a.with_ids)
+            CK(cudaMemcpyAsync(a.ckpt_ids + (size_t)j * n_pad, ctx->agents.ids, n_pad * sizeof(uint32_t),
+                               cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing ids");
+        CK(cudaMemcpyAsync(a.ckpt_trail + (size_t)j * cells, ctx->trail[ctx->cur], cells * sizeof(float),
+                           cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing trail");
+        uint32_t m = (n_steps - j * K) < K ? (n_steps - j * K) : K;
+        while (m > 0) {
+            const bool marks = use_marks(ctx);
+            if ((rc = prepare_deposits(ctx, marks)) != SLIME_OK) return rc;
+            const uint32_t chunk = ctx->opt.graph_chunk ? ctx->opt.graph_chunk : 50;
+            const uint32_t take = m < chunk ? m : chunk;
+            rc = ctx->opt.use_graphs ? run_steps_graph(ctx, take, marks) : run_steps_direct(ctx, take, marks);
+            if (rc != SLIME_OK) return rc;
+            after_steps(ctx, marks, take);
+            m -= take;
+        }
+    }
+    return SLIME_OK;
+}
+
+} // namespace
+
 extern "C" {
 
 int slime_forward_record(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) {
@@ -197,52 +509,23 @@ int slime_forward_record(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) 
         return set_error(ctx->err, SLIME_ERR_INVALID_ARGUMENT, "n_steps and ckpt_every must be >= 1");
     cudaSetDevice(ctx->device);
     CK(cudaStreamSynchronize(ctx->stream), "forward_record");
-    free_adjoint(ctx);
-    int orc = ensure_dispatch_order(ctx);
-    if (orc != SLIME_OK) return orc;
-    auto& a = ctx->adj;
-    const size_t cells = (size_t)ctx->W * ctx->H;
-    const uint64_t n_pad = ctx->agents.n_pad;
-    const uint32_t K = ckpt_every < n_steps ? ckpt_every : n_steps;
-    a.n_steps = n_steps;
-    a.ckpt_every = K;
-    a.n_ckpt = (n_steps + K - 1) / K;
-    a.dev = ctx->dev;
-    a.tile = ctx->tile;
-    a.agent_shape = ctx->agent_shape;
-    a.rate_active = (ctx->params.diffusion_rate > 0.0f && ctx->params.diffusion_rate < 1.0f) ? 1u : 0u;
-    a.n = ctx->agents.n;
-    a.n_pad = n_pad;
-    a.with_ids = ctx->agents.ids != nullptr;
-    cudaError_t e;
-    if ((e = ctx_alloc(ctx, (void**)&a.ckpt_agents, (size_t)a.n_ckpt * 4 * n_pad * sizeof(float))) != cudaSuccess ||
-        (a.with_ids && (e = ctx_alloc(ctx, (void**)&a.ckpt_ids, (size_t)a.n_ckpt * n_pad * sizeof(uint32_t))) != cudaSuccess) ||
-        (e = ctx_alloc(ctx, (void**)&a.ckpt_trail, (size_t)a.n_ckpt * cells * sizeof(float))) != cudaSuccess) {
-        free_adjoint(ctx);
-        return cuda_error(ctx->err, e, "allocating checkpoints");
+    int rc = ensure_dispatch_order(ctx);
+    if (rc != SLIME_OK) return rc;
+    if ((rc = begin_sorted_run(ctx, n_steps)) != SLIME_OK) return rc;
+    rc = record_steps(ctx, n_steps, ckpt_every);
+    if (rc == SLIME_ERR_OUT_OF_MEMORY && ctx->in_sorted_run) {
+        // no step was made: on the context's own agents, without the copy
+        ctx->agents = ctx->own_agents;
+        ctx->in_sorted_run = false;
+        release_sorted(ctx);
+        ctx->sorted_refused = true;
+        rc = record_steps(ctx, n_steps, ckpt_every);
     }
-    for (uint32_t s = 0; s < n_steps; s++) {
-        if (s % K == 0) {
-            uint32_t j = s / K;
-            CK(cudaMemcpyAsync(a.ckpt_agents + (size_t)j * 4 * n_pad, ctx->agent_block, 4 * n_pad * sizeof(float),
-                               cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing agents");
-            if (a.with_ids)
-                CK(cudaMemcpyAsync(a.ckpt_ids + (size_t)j * n_pad, ctx->agents.ids, n_pad * sizeof(uint32_t),
-                                   cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing ids");
-            CK(cudaMemcpyAsync(a.ckpt_trail + (size_t)j * cells, ctx->trail[ctx->cur], cells * sizeof(float),
-                               cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing trail");
-        }
-        const bool marks = use_marks(ctx);
-        int prc = prepare_deposits(ctx, marks);
-        if (prc != SLIME_OK) return prc;
-        CK(enqueue_step(ctx, marks, false), "recording a step");
-        after_steps(ctx, marks, 1);
-        ctx->launches += kernels_per_step(ctx, marks);
-        ctx->steps_done++;
-    }
-    ctx->last_counts_valid = true;
+    const int end = end_sorted_run(ctx);
+    if (rc != SLIME_OK) return rc;
+    if (end != SLIME_OK) return end;
     CK(cudaStreamSynchronize(ctx->stream), "forward_record");
-    a.recorded = true;
+    ctx->adj.recorded = true;
     return SLIME_OK;
 }
 
@@ -256,21 +539,38 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
     const size_t cells = (size_t)ctx->W * ctx->H;
     const uint32_t K = a.ckpt_every;
     cudaError_t e;
-    if (!a.seg_trail) {
+    const size_t stride = segment_stride(ctx);
+    const uint32_t blocks = adjoint_blocks(ctx->W, ctx->H);
+    const size_t acc_bytes = (4 + 3 * kSumBlocks) * sizeof(double) + (size_t)blocks * 3 * kThreads * sizeof(float2);
+    if (!a.agents_tmp) {
         // W + 2 zero floats past the last trail: the sampler's discarded taps
-        if ((e = ctx_alloc(ctx, (void**)&a.seg_trail, ((size_t)K * cells + ctx->W + 2) * sizeof(float))) != cudaSuccess ||
-            (e = cudaMemset(a.seg_trail, 0, ((size_t)K * cells + ctx->W + 2) * sizeof(float))) != cudaSuccess ||
-            (e = ctx_alloc(ctx, (void**)&a.seg_counts, (size_t)K * cells * sizeof(uint32_t))) != cudaSuccess ||
-            (e = ctx_alloc(ctx, (void**)&a.g[0], cells * sizeof(float))) != cudaSuccess ||
-            (e = ctx_alloc(ctx, (void**)&a.g[1], cells * sizeof(float))) != cudaSuccess ||
-            (e = ctx_alloc(ctx, (void**)&a.acc, 4 * sizeof(double))) != cudaSuccess ||
-            (e = ctx_alloc(ctx, (void**)&a.agents_tmp, 4 * a.n_pad * sizeof(float))) != cudaSuccess ||
-            (a.with_ids && (e = ctx_alloc(ctx, (void**)&a.ids_tmp, a.n_pad * sizeof(uint32_t))) != cudaSuccess))
+        const size_t trail_bytes = ((size_t)K * stride + ctx->W + 2) * sizeof(float);
+        if ((e = ctx_alloc(ctx, (void**)&a.seg_trail, trail_bytes)) == cudaSuccess &&
+            (e = cudaMemsetAsync(a.seg_trail, 0, trail_bytes, ctx->stream)) == cudaSuccess &&
+            (e = ctx_alloc(ctx, (void**)&a.seg_counts, (size_t)K * stride * sizeof(uint32_t))) == cudaSuccess &&
+            (e = ctx_alloc(ctx, (void**)&a.g[0], cells * sizeof(float))) == cudaSuccess &&
+            (e = ctx_alloc(ctx, (void**)&a.g[1], cells * sizeof(float))) == cudaSuccess &&
+            (e = ctx_alloc(ctx, (void**)&a.acc, acc_bytes)) == cudaSuccess &&
+            (!a.with_ids || (e = ctx_alloc(ctx, (void**)&a.ids_tmp, a.n_pad * sizeof(uint32_t))) == cudaSuccess))
+            e = ctx_alloc(ctx, (void**)&a.agents_tmp, 4 * a.n_pad * sizeof(float));
+        if (e != cudaSuccess) {
+            // what was allocated goes back: a later call starts anew
+            void** ptrs[] = {(void**)&a.seg_trail, (void**)&a.seg_counts, (void**)&a.g[0], (void**)&a.g[1],
+                             (void**)&a.acc, (void**)&a.ids_tmp, (void**)&a.agents_tmp};
+            for (void** q : ptrs) {
+                dev_free(*q);
+                *q = nullptr;
+            }
             return cuda_error(ctx->err, e, "allocating adjoint buffers");
+        }
+        for (uint32_t i = 0; i < K && agent_shape_uses_texture(a.agent_shape); i++)
+            a.seg_tex.push_back(make_trail_texture(a.seg_trail + i * stride, ctx->W, ctx->H));
     }
     CK(cudaMemcpyAsync(a.g[0], dl_dtrail_final, cells * sizeof(float), cudaMemcpyHostToDevice, ctx->stream),
        "uploading dL/dT");
-    CK(cudaMemsetAsync(a.acc, 0, 4 * sizeof(double), ctx->stream), "clearing gradients");
+    CK(cudaMemsetAsync(a.acc, 0, acc_bytes, ctx->stream), "clearing gradients");
+    double* parts = (double*)a.acc;                      // 3, then 3 x kSumBlocks, then every thread's
+    float2* thread_acc = (float2*)(parts + 4 + 3 * kSumBlocks);
     int cg = 0;
     AgentsSoA tmp;
     tmp.x = a.agents_tmp;
@@ -286,16 +586,20 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
     // once per (m, g0) as a CUDA graph and replayed.
     auto enqueue_segment = [&](uint32_t m, int g0) -> cudaError_t {
         cudaError_t ce = cudaSuccess;
+        const bool strips = trail_tile_streams(a.dev, a.tile);
         for (uint32_t i = 0; i < m && ce == cudaSuccess; i++) {
-            float* Ti = a.seg_trail + (size_t)i * cells;
-            uint32_t* Ki = a.seg_counts + (size_t)i * cells;
-            ce = launch_agents(a.dev, tmp, Ti, Ki, ctx->stream, a.agent_shape);
-            if (ce == cudaSuccess && i + 1 < m) ce = launch_trail(a.dev, a.tile, Ti, Ki, Ti + cells, nullptr, ctx->stream);
+            float* Ti = a.seg_trail + (size_t)i * stride;
+            uint32_t* Ki = a.seg_counts + (size_t)i * stride;
+            ce = launch_agents(a.dev, tmp, Ti, Ki, ctx->stream, a.agent_shape, nullptr,
+                               i < a.seg_tex.size() ? a.seg_tex[i] : 0, nullptr, i > 0 && strips);
+            if (ce == cudaSuccess && i + 1 < m)
+                ce = launch_trail(a.dev, a.tile, Ti, Ki, Ti + stride, nullptr, ctx->stream, nullptr, a.n > 0);
         }
         int gi = g0;
         for (int64_t i = (int64_t)m - 1; i >= 0 && ce == cudaSuccess; i--) {
-            ce = launch_adjoint_step(a.dev, a.seg_trail + (size_t)i * cells, a.seg_counts + (size_t)i * cells, a.g[gi],
-                                     a.g[1 - gi], a.acc, a.rate_active, ctx->stream);
+            // the first backward step follows the replay, the others each other
+            ce = launch_adjoint_step(a.dev, a.seg_trail + (size_t)i * stride, a.seg_counts + (size_t)i * stride,
+                                     a.g[gi], a.g[1 - gi], thread_acc, a.rate_active, ctx->stream, i + 1 < (int64_t)m);
             gi = 1 - gi;
         }
         return ce;
@@ -329,7 +633,7 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
                                cudaMemcpyDeviceToDevice, ctx->stream), "restoring ids");
         CK(cudaMemcpyAsync(a.seg_trail, a.ckpt_trail + (size_t)j * cells, cells * sizeof(float),
                            cudaMemcpyDeviceToDevice, ctx->stream), "restoring trail");
-        CK(cudaMemsetAsync(a.seg_counts, 0, (size_t)m * cells * sizeof(uint32_t), ctx->stream), "clearing counts");
+        CK(cudaMemsetAsync(a.seg_counts, 0, (size_t)m * stride * sizeof(uint32_t), ctx->stream), "clearing counts");
         cudaGraphExec_t exec = segment_graph(m, cg);
         if (exec)
             CK(cudaGraphLaunch(exec, ctx->stream), "launching a backward segment");
@@ -338,8 +642,12 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
         ctx->launches += (uint64_t)m * agent_pass_kernels(a.dev, a.n, false) + (m - 1) + m;
         if (m & 1) cg = 1 - cg;
     }
-    double acc[4];
-    CK(cudaMemcpyAsync(acc, a.acc, 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream), "reading gradients");
+    sum_threads_kernel<<<dim3(kSumBlocks, 3), kThreads, 0, ctx->stream>>>(thread_acc, blocks, parts + 4);
+    sum_parts_kernel<<<3, kThreads, 0, ctx->stream>>>(parts + 4, parts);
+    CK(cudaGetLastError(), "summing gradients");
+    ctx->launches += 2;
+    double acc[3];
+    CK(cudaMemcpyAsync(acc, parts, 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream), "reading gradients");
     if (d_trail0)
         CK(cudaMemcpyAsync(d_trail0, a.g[cg], cells * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream),
            "reading dL/dT0");

@@ -5,6 +5,7 @@
 #include <map>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "kernels.h"
 
@@ -111,10 +112,11 @@ struct slime_ctx {
         float* ckpt_agents = nullptr;     // n_ckpt * 4 * n_pad floats
         uint32_t* ckpt_ids = nullptr;     // n_ckpt * n_pad (when reordered)
         float* ckpt_trail = nullptr;      // n_ckpt * cells
-        float* seg_trail = nullptr;       // ckpt_every * cells: T_s of the segment being replayed
-        uint32_t* seg_counts = nullptr;   // ckpt_every * cells: k_s
+        float* seg_trail = nullptr;       // T_s of the segment being replayed, one every 64-float-aligned cells
+        uint32_t* seg_counts = nullptr;   // k_s, likewise
+        std::vector<cudaTextureObject_t> seg_tex; // gather textures over the T_s (0 = none)
         float* g[2] = {nullptr, nullptr}; // dL/dT ping-pong
-        double* acc = nullptr;            // d_decay, d_rate, d_dep
+        void* acc = nullptr;              // d_decay, d_rate, d_dep, and the sums they are made from
         float* agents_tmp = nullptr;      // replay copy of the agents (4 * n_pad)
         uint32_t* ids_tmp = nullptr;
         // captured segments (replay and backward steps) by (steps, g buffer)
@@ -141,6 +143,8 @@ uint64_t kernels_per_step(const slime_ctx* ctx, bool marks);
 // the agents it updates first.
 int ensure_dispatch_order(slime_ctx* ctx);
 int run_steps(slime_ctx* ctx, uint32_t n);
+int run_steps_direct(slime_ctx* ctx, uint32_t m, bool marks);
+int run_steps_graph(slime_ctx* ctx, uint32_t m, bool marks);
 int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps);
 int resort_run(slime_ctx* ctx);
 int end_sorted_run(slime_ctx* ctx);

@@ -127,11 +127,12 @@ int trail_tma_misaligned_blocks();
 // ---- adjoint.cu
 // One backward step of the frozen-trajectory chain: from g_in = dL/dT_{s+1}
 // and the step's input trail T_s and counts k_s, writes g_out = dL/dT_s and
-// adds the step's parameter-gradient contributions to acc[0..2]
-// (decay_factor, diffusion_rate, deposition), in binary64.
+// adds the step's parameter-gradient contributions to every thread's own sums
+// in acc (decay_factor, diffusion_rate, deposition).  With `pdl` it follows
+// another backward step, and its T and k were complete before that one began.
 cudaError_t launch_adjoint_step(const DevParams& p, const float* trail_s, const uint32_t* counts_s,
-                                const float* g_in, float* g_out, double* acc, uint32_t rate_active,
-                                cudaStream_t s);
+                                const float* g_in, float* g_out, float2* acc, uint32_t rate_active,
+                                cudaStream_t s, bool pdl);
 
 // ---- reorder.cu
 // Morton reordering of agent slots by cell through scratch buffers; keeps ids.

@@ -110,7 +110,9 @@ __device__ __noinline__ GroupState<APT> step_partial_group(const DevParams& p, G
 // A thread moves APT consecutive slots with one vector load/store per field.
 // MINB > 0 asks the compiler to fit MINB blocks per SM (caps registers).
 // Trail is the reader of the sensed trail (TrailPtr or TrailTex).
-template <int APT, int BS, int MINB, bool kIds, class Trail>
+// With kLate the launch follows a kernel that only clears the deposit record: it
+// waits for that just before its deposits.
+template <int APT, int BS, int MINB, bool kIds, class Trail, bool kLate = false>
 __global__ void __launch_bounds__(BS, MINB) agents_kernel(const __grid_constant__ DevParams p, float* __restrict__ X,
                                                     float* __restrict__ Y, float* __restrict__ TH,
                                                     float* __restrict__ V, const uint32_t* __restrict__ ids,
@@ -133,8 +135,10 @@ __global__ void __launch_bounds__(BS, MINB) agents_kernel(const __grid_constant_
     }
     // the state is not written by the trail pass this launch may follow; the
     // trail it senses and the deposit record are
-    pdl_wait();
-    pdl_trigger();
+    if (!kLate) {
+        pdl_wait();
+        pdl_trigger();
+    }
     int cell[APT];
     if (base + APT <= n) {
         // full group: no per-agent branch, so the agents' work can interleave
@@ -144,6 +148,10 @@ __global__ void __launch_bounds__(BS, MINB) agents_kernel(const __grid_constant_
         for (int j = 0; j < APT; j++)
             cell[j] = (base + j < n) ? agent_step(p, x[j], y[j], th[j], v[j], (int32_t)id[j], trail) : -1;
     }
+    if (kLate) {
+        pdl_wait();
+        pdl_trigger();
+    }
 #pragma unroll
     for (int j = 0; j < APT; j++)
         if (cell[j] >= 0) deposit(counts, marks, cell[j]);
@@ -151,6 +159,25 @@ __global__ void __launch_bounds__(BS, MINB) agents_kernel(const __grid_constant_
     Lanes<APT>::store(Y + base, y);
     Lanes<APT>::store(TH + base, th);
     Lanes<APT>::store(V + base, v);
+}
+
+__global__ void __launch_bounds__(256) clear_counts_kernel(uint32_t* __restrict__ counts, uint32_t cells) {
+    // the agent pass after it may start: it clears nothing that pass reads
+    // before its own wait
+    pdl_trigger();
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    if (((uintptr_t)counts & 15) == 0) {
+        const uint32_t at = 4 * i;
+        if (at + 4 <= cells) *reinterpret_cast<uint4*>(counts + at) = make_uint4(0u, 0u, 0u, 0u);
+        else
+            for (uint32_t j = at; j < cells; j++) counts[j] = 0u;
+    } else {
+        // every 256 of a block's 1024 words consecutive over its threads
+        for (uint32_t j = 0; j < 4; j++) {
+            const uint32_t at = blockIdx.x * 1024 + j * 256 + threadIdx.x;
+            if (at < cells) counts[at] = 0u;
+        }
+    }
 }
 
 __global__ void aos_to_soa_kernel(const float4* __restrict__ aos, float* __restrict__ x, float* __restrict__ y,
@@ -467,6 +494,27 @@ cudaError_t launch_recount(const DevParams& p, const AgentsSoA& a, uint32_t* cou
     uint32_t wy = 0, span = 0;
     if (p.dispatch_mode == SLIME_DISPATCH_REFERENCE) slm_dispatch_geometry(a.n, &wy, &span);
     recount_kernel<<<blocks_for(a.n, 256), 256, 0, s>>>(a.x, a.y, a.ids, a.n, p.W, p.H, wy, span, counts);
+    return cudaGetLastError();
+}
+
+// One pass over caller-owned arrays in no order (ids are slots, nothing padded),
+// with the counts cleared first.
+cudaError_t launch_agents_caller(const DevParams& p, const AgentsSoA& a, const float* trail, uint32_t* counts,
+                                 cudaStream_t s) {
+    const uint32_t cells = (uint32_t)((uint64_t)p.W * p.H);
+    clear_counts_kernel<<<(cells + 1023) / 1024, 256, 0, s>>>(counts, cells);
+    cudaError_t e = cudaGetLastError();
+    AgentsSoA now = a;
+    if (p.dispatch_mode == SLIME_DISPATCH_REFERENCE) now.n = reference_dispatch_updated(a.n);
+    if (e != cudaSuccess || now.n == 0) return e;
+    const dim3 grid(blocks_for(now.n, 256));
+    e = launch_kp(agents_kernel<1, 256, 0, false, TrailPtr, true>, grid, dim3(256), 0, s, nullptr, true, p, now.x, now.y,
+                  now.th, now.v, (const uint32_t*)nullptr, TrailPtr{trail}, counts, (uint8_t*)nullptr, (uint32_t)now.n,
+                  now.n);
+    if (e != cudaSuccess || agent_pass_kernels(p, a.n, false) == 1) return e;
+    uint32_t wy = 0, span = 0;
+    slm_dispatch_geometry(a.n, &wy, &span);
+    extra_deposits_kernel<<<blocks_for(now.n, 256), 256, 0, s>>>(now.x, now.y, nullptr, now.n, p.W, p.H, wy, span, counts);
     return cudaGetLastError();
 }
 

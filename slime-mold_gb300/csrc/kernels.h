@@ -48,6 +48,10 @@ int agent_shape_default(uint64_t n, bool tex);
 cudaError_t launch_agents(const DevParams& p, const AgentsSoA& a, const float* trail, uint32_t* counts,
                           cudaStream_t s, int shape = 0, const cudaAccessPolicyWindow* win = nullptr,
                           cudaTextureObject_t tex = 0, uint8_t* marks = nullptr, bool pdl = false);
+// The same over caller-owned arrays, one agent per thread and ids the slots,
+// after clearing `counts`.
+cudaError_t launch_agents_caller(const DevParams& p, const AgentsSoA& a, const float* trail, uint32_t* counts,
+                                 cudaStream_t s);
 // Kernels one launch_agents call enqueues.
 int agent_pass_kernels(const DevParams& p, uint64_t n, bool marks);
 // How many agents (ids 0 .. this - 1) the reference's dispatch updates.
@@ -75,6 +79,8 @@ TrailTile trail_tile(int index);
 // marks or counts; with `aligned` false one that reads and writes buffers of
 // any alignment.
 int trail_tile_default(const DevParams& p, bool marks, bool aligned = true);
+// The 8-row streaming tile, or -1 where it cannot run.
+int trail_tile_strips(const DevParams& p);
 // Whether tile `index` can run this parameter set / grid (the streaming
 // tiles need W % 4 == 0 and a blur radius of 1 or 2).
 bool trail_tile_supported(const DevParams& p, int tile);

@@ -56,10 +56,6 @@ int step_with_counts(const SlimeParams* params, uint32_t width, uint32_t height,
     DevParams d;
     const char* why = nullptr;
     if (!make_dev_params(*params, width, height, &d, &why)) return SLIME_ERR_INVALID_ARGUMENT;
-    if (cudaMemsetAsync(counts, 0, cells * sizeof(uint32_t), s) != cudaSuccess) {
-        cudaGetLastError();
-        return SLIME_ERR_CUDA;
-    }
     AgentsSoA a;
     a.x = d_x;
     a.y = d_y;
@@ -68,13 +64,18 @@ int step_with_counts(const SlimeParams* params, uint32_t width, uint32_t height,
     a.ids = nullptr;
     a.n = n_agents;
     a.n_pad = n_agents;
-    // One agent per thread (scalar loads need no padding or 16-byte
-    // alignment of the caller's arrays); the trail pass of unaligned trails or
-    // counts is a shared-memory tile.
-    const int kScalarShape = 2;
-    cudaError_t e = launch_agents(d, a, d_trail_in, counts, s, kScalarShape, nullptr);
+    // One agent per thread: scalar loads need no padding or 16-byte alignment of
+    // the caller's arrays.  The count clear, the agent pass and the trail pass
+    // are a chain of programmatic dependents, each started while the one before
+    // finishes.  The trail pass is streaming strips (no shared-memory carve-out,
+    // see trail_tile.cuh), and of unaligned trails or counts, or other widths and
+    // radii, a shared-memory tile.
+    cudaError_t e = launch_agents_caller(d, a, d_trail_in, counts, s);
     const bool aligned = (((uintptr_t)d_trail_in | (uintptr_t)d_trail_out | (uintptr_t)counts) & 15) == 0;
-    if (e == cudaSuccess) e = launch_trail(d, trail_tile_default(d, false, aligned), d_trail_in, counts, d_trail_out, nullptr, s, nullptr);
+    const int strips = trail_tile_strips(d);
+    const int tile = aligned && strips >= 0 ? strips : trail_tile_default(d, false, aligned);
+    if (e == cudaSuccess)
+        e = launch_trail(d, tile, d_trail_in, counts, d_trail_out, nullptr, s, nullptr, n_agents > 0);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return SLIME_ERR_CUDA;

@@ -98,6 +98,7 @@ int trail_tile_default(const DevParams& p, bool marks, bool aligned) {
     if (aligned && cells >= strips_from && trail_tile_supported(p, kNumTiles)) return kNumTiles;
     return cells < 2000000 || (gauss && p.R == 1) ? 4 : 5;
 }
+int trail_tile_strips(const DevParams& p) { return trail_tile_supported(p, kNumTiles) ? kNumTiles : -1; }
 bool trail_tile_supported(const DevParams& p, int tile) {
     if (tile == kTrailTileTma) return trail_tma_supported(p);
     if (tile < 0 || tile >= kNumTiles + kNumStream) return false;

@@ -575,14 +575,15 @@ SLM_FN uint32_t slm_dispatch_visits(uint64_t n, uint64_t index) {
 /* slm_sincos of two arguments with |x0|, |x1| < 4096 at once, bit for bit.
  * Each lane's reduction starts with a binary32 product and sum (a packed
  * product followed by a packed sum may be contracted into one fused
- * operation, which would round once instead of twice, so these stay
+ * operation, which would round once instead of twice, so the sums stay
  * scalar); every later step is a fused multiply-add, or a product that feeds
  * one as a multiplicand, evaluated for both lanes by one packed instruction
  * (fma.rn.f32x2, mul.rn.f32x2: each lane rounded as its scalar form). */
 static __device__ __forceinline__ void slm_sincos2_cw(float x0, float x1, float* s0, float* c0, float* s1,
                                                       float* c1) {
-    const float b0 = slm_add(slm_mul(x0, SLM_TWO_OVER_PI_F), 12582912.0f);
-    const float b1 = slm_add(slm_mul(x1, SLM_TWO_OVER_PI_F), 12582912.0f);
+    const float2 m = __fmul2_rn(make_float2(x0, x1), make_float2(SLM_TWO_OVER_PI_F, SLM_TWO_OVER_PI_F));
+    const float b0 = slm_add(m.x, 12582912.0f);
+    const float b1 = slm_add(m.y, 12582912.0f);
     /* -j, exactly: 1.5 * 2^23 - biased, as one packed sum (a packed sum of
      * operands that no packed product produced rounds per lane) */
     const float2 nj = __fadd2_rn(make_float2(12582912.0f, 12582912.0f), make_float2(-b0, -b1));
@@ -730,7 +731,10 @@ static __device__ __forceinline__ void slm_jitter_hash2(int32_t i0, float x0, fl
                                                         float y1, float* h0, float* h1) {
     float r0, r1, s0, c0, s1, c1;
     int q0, q1;
-    const float a0 = slm_jitter_arg(i0, x0, y0), a1 = slm_jitter_arg(i1, x1, y1);
+    const float2 mi = __fmul2_rn(make_float2(slm_i2f(i0), slm_i2f(i1)), make_float2(12.9898f, 12.9898f));
+    const float2 mx = __fmul2_rn(make_float2(x0, x1), make_float2(78.233f, 78.233f));
+    const float2 my = __fmul2_rn(make_float2(y0, y1), make_float2(37.719f, 37.719f));
+    const float a0 = slm_add(slm_add(mi.x, mx.x), my.x), a1 = slm_add(slm_add(mi.y, mx.y), my.y);
     const uint32_t e0 = ((slm_f2u_bits(a0) >> 23) & 0xffu) - 139u, e1 = ((slm_f2u_bits(a1) >> 23) & 0xffu) - 139u;
     if (e0 <= 31u && e1 <= 31u) {
         slm_reduce_pio2_win(a0, &r0, &q0);
@@ -740,8 +744,9 @@ static __device__ __forceinline__ void slm_jitter_hash2(int32_t i0, float x0, fl
         r0 = o.a.r, q0 = o.a.q, r1 = o.b.r, q1 = o.b.q;
     }
     slm_sincos_rq2(r0, q0, r1, q1, &s0, &c0, &s1, &c1);
-    *h0 = slm_fract(slm_mul(s0, 43758.5453f));
-    *h1 = slm_fract(slm_mul(s1, 43758.5453f));
+    const float2 ms = __fmul2_rn(make_float2(s0, s1), make_float2(43758.5453f, 43758.5453f));
+    *h0 = slm_fract(ms.x);
+    *h1 = slm_fract(ms.y);
 }
 #endif
 

@@ -512,18 +512,17 @@ int slime_forward_record(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) 
     int rc = ensure_dispatch_order(ctx);
     if (rc != SLIME_OK) return rc;
     if ((rc = begin_sorted_run(ctx, n_steps)) != SLIME_OK) return rc;
+    ctx->keep_sorted = ctx->in_sorted_run;
     rc = record_steps(ctx, n_steps, ckpt_every);
+    ctx->keep_sorted = false;
     if (rc == SLIME_ERR_OUT_OF_MEMORY && ctx->in_sorted_run) {
         // no step was made: on the context's own agents, without the copy
-        ctx->agents = ctx->own_agents;
-        ctx->in_sorted_run = false;
+        if ((rc = end_sorted_run(ctx)) != SLIME_OK) return rc;
         release_sorted(ctx);
         ctx->sorted_refused = true;
         rc = record_steps(ctx, n_steps, ckpt_every);
     }
-    const int end = end_sorted_run(ctx);
     if (rc != SLIME_OK) return rc;
-    if (end != SLIME_OK) return end;
     CK(cudaStreamSynchronize(ctx->stream), "forward_record");
     ctx->adj.recorded = true;
     return SLIME_OK;

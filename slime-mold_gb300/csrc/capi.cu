@@ -333,8 +333,9 @@ namespace slime {
 // own agents) is given back first.
 cudaError_t ctx_alloc(slime_ctx* ctx, void** p, size_t bytes) {
     cudaError_t e = dev_alloc(p, bytes);
-    if (e == cudaSuccess || !ctx->sorted_block || ctx->in_sorted_run) return e;
+    if (e == cudaSuccess || !ctx->sorted_block || ctx->keep_sorted) return e;
     cudaGetLastError();
+    if (end_sorted_run(ctx) != SLIME_OK) return e;
     release_sorted(ctx);
     ctx->sorted_refused = true;
     if (!ctx->agents.ids) {
@@ -600,6 +601,8 @@ int run_steps_graph(slime_ctx* ctx, uint32_t m, bool marks) {
 
 int do_reorder(slime_ctx* ctx) {
     if (ctx->agents.n == 0) return SLIME_OK;
+    const int erc = end_sorted_run(ctx);
+    if (erc != SLIME_OK) return erc;
     if (!ctx->agents.ids) {
         CK(ctx_alloc(ctx, (void**)&ctx->ids_storage, ctx->agents.n_pad * sizeof(uint32_t)), "allocating agent ids");
         CK(cudaMemsetAsync(ctx->ids_storage, 0, ctx->agents.n_pad * sizeof(uint32_t), ctx->stream),
@@ -620,13 +623,17 @@ int do_reorder(slime_ctx* ctx) {
     return SLIME_OK;
 }
 
-// ---- runs of steps on a sorted copy of the agents.
+// ---- steps on a sorted copy of the agents.
 // A context that is not asked to reorder its agents (reorder_every 0, and
 // never reordered by hand) keeps every agent in its slot.  Steps on agents in no
 // order sense the trail at random, 32-byte sectors from L2 for every footprint.
-// So a call of several steps sorts the agents into a copy, steps the copy and
-// puts every agent back into its slot: the same results in the same slots.
-// Measured (us a step, in slot order / on a copy): 65,536 agents on 512^2, 32
+// So once enough steps are to be made, or were made one by one, the agents are
+// sorted into a copy that is stepped in their place (`agents`, with the id of
+// every slot) until something needs them in their slots: reordering by hand or
+// by schedule, the reference's dispatch, the autotuner, a resize.  Reading them
+// back does not (records go out in id order either way), and what replaces them
+// drops the copy.  The results are the same.
+// Measured (us a step, in slot order / on a copy, sort and return included): 65,536 agents on 512^2, 32
 // steps 6.5 / 6.9, 100 steps 6.5 / 6.1; 262,144 on 1024^2, 16 steps 13.0 / 11.7,
 // 100 12.8 / 9.0; 500,003 on 1001x777, 16 22.8 / 19.6, 100 22.6 / 17.6;
 // 1,048,576 on 1024^2, 8 33.9 / 28.9, 100 33.5 / 19.8; 10 M on 1600x900, 8
@@ -656,7 +663,8 @@ void release_sorted(slime_ctx* ctx) {
 bool sorted_run_ready(slime_ctx* ctx, uint32_t n_steps) {
     const uint64_t n = ctx->agents.n, n_pad = ctx->agents.n_pad;
     if (ctx->opt.reorder_every || ctx->agents.ids || ctx->sorted_refused ||
-        n_steps < sorted_min_steps(n) || ctx->dev.dispatch_mode != SLIME_DISPATCH_EACH_AGENT)
+        (uint64_t)n_steps + ctx->slot_steps < sorted_min_steps(n) ||
+        ctx->dev.dispatch_mode != SLIME_DISPATCH_EACH_AGENT)
         return false;
     if (!ctx->sorted_block) {
         const size_t bytes = 5 * n_pad * sizeof(float);
@@ -673,7 +681,10 @@ bool sorted_run_ready(slime_ctx* ctx, uint32_t n_steps) {
     return true;
 }
 
+// Before n_steps steps: onto the copy where that pays, the copy sorted again
+// where its order has aged.
 int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps) {
+    if (ctx->in_sorted_run) return resort_run(ctx);
     if (!sorted_run_ready(ctx, n_steps)) return SLIME_OK;
     AgentsSoA to = ctx->agents;
     to.x = (float*)ctx->sorted_block;
@@ -697,7 +708,7 @@ int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps) {
     return SLIME_OK;
 }
 
-// Between steps of a sorted run: sort the copy again when its order has aged.
+// Between steps on the copy: sort it again when its order has aged.
 int resort_run(slime_ctx* ctx) {
     if (!ctx->in_sorted_run || ctx->steps_done - ctx->sorted_since < sorted_steps(ctx)) return SLIME_OK;
     CK(launch_reorder(ctx->agents, ctx->agents, ctx->W, ctx->H, 2, ctx->reorder, ctx->stream), "sorting agents");
@@ -706,13 +717,20 @@ int resort_run(slime_ctx* ctx) {
     return SLIME_OK;
 }
 
+// The context's own agents again, with what they were when the copy was made:
+// for what is about to overwrite them.
+void drop_sorted_run(slime_ctx* ctx) {
+    if (ctx->in_sorted_run) ctx->agents = ctx->own_agents;
+    ctx->in_sorted_run = false;
+    ctx->slot_steps = 0;
+}
+
 // Every agent back into its own slot (by way of the sort scratch, as one
 // 16-byte record an agent).
 int end_sorted_run(slime_ctx* ctx) {
     if (!ctx->in_sorted_run) return SLIME_OK;
     const AgentsSoA copy = ctx->agents;
-    ctx->agents = ctx->own_agents;
-    ctx->in_sorted_run = false;
+    drop_sorted_run(ctx);
     CK(launch_soa_to_aos(copy, (float4*)ctx->reorder.buf, ctx->stream), "unsorting agents");
     CK(launch_aos_to_soa((const float4*)ctx->reorder.buf, ctx->agents, ctx->stream), "unsorting agents");
     ctx->launches += 2;
@@ -807,10 +825,10 @@ int ensure_dispatch_order(slime_ctx* ctx) {
 // run_steps: graph_chunk steps, cut at reorder boundaries), without stepping.
 int prepare_steps(slime_ctx* ctx, uint32_t n) {
     if (!ctx->opt.use_graphs || ctx->agents.n == 0) return SLIME_OK;
-    int brc = begin_sorted_run(ctx, n); // graphs of a sorted run step the copy
+    int brc = begin_sorted_run(ctx, n); // the graphs step the copy, then
     if (brc != SLIME_OK) return brc;
     const uint32_t aged = ctx->in_sorted_run ? sorted_steps(ctx) : ~0u;
-    uint32_t age = 0;
+    uint32_t age = ctx->in_sorted_run ? (uint32_t)(ctx->steps_done - ctx->sorted_since) : 0u;
     const bool marks = use_marks(ctx);
     const uint32_t chunk = ctx->opt.graph_chunk ? ctx->opt.graph_chunk : 50;
     const int saved = ctx->cur;
@@ -833,10 +851,6 @@ int prepare_steps(slime_ctx* ctx, uint32_t n) {
         n -= take;
     }
     ctx->cur = saved;
-    if (ctx->in_sorted_run) { // nothing was stepped
-        ctx->agents = ctx->own_agents;
-        ctx->in_sorted_run = false;
-    }
     return rc;
 }
 
@@ -876,9 +890,8 @@ int run_steps(slime_ctx* ctx, uint32_t n) {
     int rc;
     if ((rc = ensure_dispatch_order(ctx)) != SLIME_OK) return rc;
     if ((rc = begin_sorted_run(ctx, n)) != SLIME_OK) return rc;
-    rc = run_steps_on(ctx, n);
-    const int end = end_sorted_run(ctx);
-    return rc != SLIME_OK ? rc : end;
+    if (!ctx->in_sorted_run) ctx->slot_steps += n;
+    return run_steps_on(ctx, n);
 }
 
 } // namespace slime
@@ -983,6 +996,10 @@ int slime_set_params(slime_ctx* ctx, const SlimeParams* params) {
     ctx->params.width = ctx->W;
     ctx->params.height = ctx->H;
     if (memcmp(&d, &ctx->dev, sizeof d) != 0) {
+        if (d.dispatch_mode != SLIME_DISPATCH_EACH_AGENT) {
+            const int rc = end_sorted_run(ctx);
+            if (rc != SLIME_OK) return rc;
+        }
         ctx->dev = d;
         invalidate_graphs(ctx); // the parameter block is baked into the captured launches
         choose_kernels(ctx);
@@ -1006,6 +1023,10 @@ int slime_set_options(slime_ctx* ctx, const SlimeOptions* o) {
     if (o->agent_shape > (uint32_t)agent_shape_count())
         return set_error(ctx->err, SLIME_ERR_INVALID_ARGUMENT, "agent_shape out of range (0..%d)",
                          agent_shape_count());
+    if (o->reorder_every) {
+        const int rc = end_sorted_run(ctx);
+        if (rc != SLIME_OK) return rc;
+    }
     const bool l2_changed = (o->l2_persist != 0) != (ctx->opt.l2_persist != 0);
     ctx->opt = *o;
     if (ctx->opt.graph_chunk == 0) ctx->opt.graph_chunk = 50;
@@ -1053,6 +1074,7 @@ int slime_upload_agents(slime_ctx* ctx, const float* aos, uint64_t n) {
     int rc;
     if ((rc = make_counts(ctx)) != SLIME_OK) return rc;
     if ((rc = ensure_staging(ctx, n * sizeof(float4))) != SLIME_OK) return rc;
+    drop_sorted_run(ctx);
     CK(cudaMemcpyAsync(ctx->staging, aos, n * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream), "uploading agents");
     CK(launch_aos_to_soa((const float4*)ctx->staging, ctx->agents, ctx->stream), "converting agents");
     if ((rc = reset_ids(ctx)) != SLIME_OK) return rc;
@@ -1080,6 +1102,7 @@ int slime_seed_agents(slime_ctx* ctx, uint64_t seed, float hmin, float hmax) {
     cudaSetDevice(ctx->device);
     int rc = make_counts(ctx);
     if (rc != SLIME_OK) return rc;
+    drop_sorted_run(ctx);
     CK(launch_seed_agents(ctx->agents, seed, (float)ctx->W, (float)ctx->H, hmin, hmax, ctx->params.agent_speed_min,
                           ctx->params.agent_speed_max, ctx->stream),
        "seeding agents");
@@ -1146,6 +1169,7 @@ int slime_resize(slime_ctx* ctx, uint32_t width, uint32_t height) {
     DevParams d;
     const char* why = nullptr;
     if (!make_dev_params(np, width, height, &d, &why)) return set_error(ctx->err, SLIME_ERR_INVALID_ARGUMENT, "%s", why);
+    if ((rc = end_sorted_run(ctx)) != SLIME_OK) return rc;
     CK(cudaStreamSynchronize(ctx->stream), "resizing");
     // the graphs and the adjoint recording belong to the old size; the new
     // trails replace the old only once allocated, so a resize that runs out
@@ -1153,6 +1177,7 @@ int slime_resize(slime_ctx* ctx, uint32_t width, uint32_t height) {
     invalidate_graphs(ctx);
     free_adjoint(ctx);
     release_sorted(ctx);
+    ctx->sorted_refused = false;
     if ((rc = alloc_trail(ctx, width, height)) != SLIME_OK) return rc;
     // src/main.rs:987-993: scale = new / old as f32 division.
     float sx = slm_div((float)width, (float)ctx->W);
@@ -1177,6 +1202,7 @@ int slime_set_agent_count(slime_ctx* ctx, uint64_t n, uint64_t seed) {
     int rc;
     if ((rc = valid_size(ctx->err, ctx->W, ctx->H, n)) != SLIME_OK) return rc;
     if ((rc = make_counts(ctx)) != SLIME_OK) return rc;
+    if ((rc = end_sorted_run(ctx)) != SLIME_OK) return rc; // out of memory, they stay
     CK(cudaStreamSynchronize(ctx->stream), "changing the agent count");
     // the new block replaces the agents only once allocated: out of memory,
     // the context keeps its agents
@@ -1193,6 +1219,7 @@ int slime_set_agent_count(slime_ctx* ctx, uint64_t n, uint64_t seed) {
 
 int slime_set_steps_done(slime_ctx* ctx, uint64_t steps_done) {
     if (!ctx) return SLIME_ERR_INVALID_ARGUMENT;
+    ctx->sorted_since += steps_done - ctx->steps_done; // the sorted copy's age stays
     ctx->steps_done = steps_done;
     // no reorder has happened at this count yet: one falls due here when
     // steps_done is a multiple of reorder_every, as in the run being resumed
@@ -1475,6 +1502,8 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
     if (!ctx) return SLIME_ERR_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
     if (reps == 0) reps = 5;
+    const int erc = end_sorted_run(ctx);
+    if (erc != SLIME_OK) return erc;
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0), "creating events");
     CK(cudaEventCreate(&e1), "creating events");

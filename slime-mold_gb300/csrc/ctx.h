@@ -25,13 +25,15 @@ struct slime_ctx {
     uint64_t reorders_done = 0;
     slime::ReorderScratch reorder;
 
-    // A run of steps on a sorted copy of the agents (capi.cu): the copy's block
-    // (x | y | angle | speed | id, n_pad each), and the context's own agents
-    // while `agents` is the copy.
+    // Steps on a sorted copy of the agents (capi.cu): the copy's block (x | y |
+    // angle | speed | id, n_pad each), and the context's own agents while `agents`
+    // is the copy.
     void* sorted_block = nullptr;
     bool sorted_refused = false; // it did not fit: not tried again for these agents
+    bool keep_sorted = false;    // a recording allocates for the copy
     bool in_sorted_run = false;
-    uint64_t sorted_since = 0; // steps_done at its last sort
+    uint64_t slot_steps = 0;   // steps made in slot order since the agents were set
+    uint64_t sorted_since = 0; // steps_done at the copy's last sort
     slime::AgentsSoA own_agents;
 
     float* trail[2] = {nullptr, nullptr};
@@ -148,6 +150,7 @@ int run_steps_graph(slime_ctx* ctx, uint32_t m, bool marks);
 int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps);
 int resort_run(slime_ctx* ctx);
 int end_sorted_run(slime_ctx* ctx);
+void drop_sorted_run(slime_ctx* ctx);
 void release_sorted(slime_ctx* ctx);
 cudaError_t ctx_alloc(slime_ctx* ctx, void** p, size_t bytes);
 // Steps after which a sorted copy is sorted again.

@@ -644,11 +644,13 @@ uint32_t sorted_min_steps(uint64_t n) { return n >= 200000 ? 16u : (n >= 32768 ?
 // The copy is sorted again when the fastest agents have crossed 32 cells (100
 // steps of 10 M agents at 0.48 cells a step: 8 cells 151.7, 16 148.3, 32 146.5,
 // 64 149.8 us), at most every 16 steps.
-uint32_t sorted_steps(const slime_ctx* ctx) {
-    const float lo = fabsf(ctx->dev.speed_min), hi = fabsf(ctx->dev.speed_max);
-    const float move = (lo > hi ? lo : hi) * fabsf(ctx->dev.time_step); // cells a step
+uint32_t sorted_steps_of(const DevParams& d) {
+    const float lo = fabsf(d.speed_min), hi = fabsf(d.speed_max);
+    const float move = (lo > hi ? lo : hi) * fabsf(d.time_step); // cells a step
     return move >= 2.0f ? 16u : (move > 0.032f ? (uint32_t)(32.0f / move) : 1000u);
 }
+
+uint32_t sorted_steps(const slime_ctx* ctx) { return sorted_steps_of(ctx->dev); }
 
 void release_sorted(slime_ctx* ctx) {
     if (!ctx->sorted_block) return;

@@ -153,7 +153,9 @@ int end_sorted_run(slime_ctx* ctx);
 void drop_sorted_run(slime_ctx* ctx);
 void release_sorted(slime_ctx* ctx);
 cudaError_t ctx_alloc(slime_ctx* ctx, void** p, size_t bytes);
-// Steps after which a sorted copy is sorted again.
+// How many steps a sort of n agents is worth, and after how many it is done again.
+uint32_t sorted_min_steps(uint64_t n);
+uint32_t sorted_steps_of(const DevParams& d);
 uint32_t sorted_steps(const slime_ctx* ctx);
 int prepare_steps(slime_ctx* ctx, uint32_t n);
 void free_adjoint(slime_ctx* ctx);

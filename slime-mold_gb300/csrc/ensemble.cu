@@ -280,6 +280,12 @@ struct slime_ensemble {
     int reorder_cell_log2 = 2;
     uint64_t steps_done = 0;
     uint64_t last_reorder_step = ~0ull;
+    // With no schedule (reorder_every 0) the colonies are sorted as a single
+    // context's copy is (capi.cu), in place: every slot has its agent's id.
+    bool auto_sort = true;
+    bool sorted = false;         // since the last upload or seed
+    uint64_t unsorted_steps = 0; // steps made without
+    uint64_t sorted_since = 0;   // steps_done at the last sort
     ReorderScratch reorder;
     ReorderScratch lane_reorder[3]; // sort scratch of the lanes engine's concurrent reorders (with `reorder`)
     float* trail[2] = {nullptr, nullptr};
@@ -555,6 +561,7 @@ cudaError_t enqueue_lane_steps(slime_ensemble* e, uint32_t m) {
 // otherwise one after another on the ensemble's stream.
 int reorder_all(slime_ensemble* e) {
     const size_t nr = e->lanes.size() < 4 ? e->lanes.size() : 4;
+    cudaError_t ce = cudaSuccess;
     if (e->engine == SLIME_ENSEMBLE_LANES && nr > 1) {
         ECK(cudaEventRecord(e->fork_ev, e->stream), "forking reorders");
         for (size_t l = 0; l < nr; l++) ECK(cudaStreamWaitEvent(e->lanes[l], e->fork_ev, 0), "forking reorders");
@@ -564,7 +571,8 @@ int reorder_all(slime_ensemble* e) {
         std::stable_sort(order.begin(), order.end(),
                          [&](uint32_t a, uint32_t b) { return e->colonies[a].n > e->colonies[b].n; });
         std::vector<uint64_t> load(nr, 0);
-        for (uint32_t j : order) {
+        for (size_t i = 0; i < order.size() && ce == cudaSuccess; i++) {
+            const uint32_t j = order[i];
             size_t l = 0;
             for (size_t k = 1; k < nr; k++)
                 if (load[k] < load[l]) l = k;
@@ -572,23 +580,54 @@ int reorder_all(slime_ensemble* e) {
             const Colony& c = e->colonies[j];
             AgentsSoA a = colony_soa(e, c);
             ReorderScratch& scratch = l == 0 ? e->reorder : e->lane_reorder[l - 1];
-            ECK(launch_reorder(a, a, c.W, c.H, e->reorder_cell_log2, scratch, e->lanes[l]), "reordering agents");
+            ce = launch_reorder(a, a, c.W, c.H, e->reorder_cell_log2, scratch, e->lanes[l]);
             e->launches += kReorderKernels;
         }
-        for (size_t l = 0; l < nr; l++) {
+        for (size_t l = 0; l < nr; l++) { // also after a failure: what was launched is waited for
             ECK(cudaEventRecord(e->lane_ev[l], e->lanes[l]), "joining reorders");
             ECK(cudaStreamWaitEvent(e->stream, e->lane_ev[l], 0), "joining reorders");
         }
     } else {
         for (const Colony& c : e->colonies) {
-            if (c.n == 0) continue;
+            if (c.n == 0 || ce != cudaSuccess) continue;
             AgentsSoA a = colony_soa(e, c);
-            ECK(launch_reorder(a, a, c.W, c.H, e->reorder_cell_log2, e->reorder, e->stream), "reordering agents");
+            ce = launch_reorder(a, a, c.W, c.H, e->reorder_cell_log2, e->reorder, e->stream);
             e->launches += kReorderKernels;
         }
     }
+    ECK(ce, "reordering agents");
     e->last_reorder_step = e->steps_done;
     return SLIME_OK;
+}
+
+// Steps after which the colonies are sorted again when no schedule says so: when
+// the fastest agents of any have crossed 32 cells.
+uint32_t ens_sorted_steps(const slime_ensemble* e) {
+    uint32_t steps = 1000;
+    for (const Colony& c : e->colonies)
+        if (c.n) steps = std::min(steps, sorted_steps_of(c.dev));
+    return steps;
+}
+
+// Before n steps: sort the colonies where that pays (the bounds of a single
+// context's copy, on the agents of all): 16 colonies of 256^2 to 1024^2 take 258
+// us a step sorted and 543 in no order.  Without scratch memory it is given up.
+int auto_sort(slime_ensemble* e, uint32_t n) {
+    if (e->reorder_every || !e->auto_sort) return SLIME_OK;
+    uint64_t agents = 0;
+    for (const Colony& c : e->colonies) agents += c.n;
+    const bool due = e->sorted ? e->steps_done - e->sorted_since >= ens_sorted_steps(e)
+                               : (uint64_t)n + e->unsorted_steps >= sorted_min_steps(agents);
+    if (!due) return SLIME_OK;
+    const int rc = reorder_all(e);
+    if (rc == SLIME_ERR_OUT_OF_MEMORY) {
+        e->auto_sort = false;
+        e->err.clear();
+        return SLIME_OK;
+    }
+    e->sorted = rc == SLIME_OK;
+    e->sorted_since = e->steps_done;
+    return rc;
 }
 
 int check_barrier(slime_ensemble* e) {
@@ -704,12 +743,19 @@ int prepare_ens_steps(slime_ensemble* e, uint32_t n) {
     int rc = prepare_ens_deposits(e);
     if (rc != SLIME_OK) return rc;
     const int saved = e->cur;
-    uint64_t steps = e->steps_done;
+    uint64_t steps = e->steps_done, agents = 0;
+    for (const Colony& c : e->colonies) agents += c.n;
+    const uint32_t aged = ens_sorted_steps(e);
+    uint32_t age = e->sorted ? (uint32_t)(e->steps_done - e->sorted_since) : 0u;
     while (n > 0) {
         uint32_t m = n < kEnsChunk ? n : kEnsChunk;
         if (e->reorder_every) {
             uint64_t to_next = e->reorder_every - steps % e->reorder_every;
             if (to_next < m) m = (uint32_t)to_next;
+        } else if (e->sorted || e->unsorted_steps + n >= sorted_min_steps(agents)) {
+            if (age >= aged) age = 0;
+            if (aged - age < m) m = aged - age;
+            age += m;
         }
         if (!chunk_graph(e, m)) break; // stepping will launch directly
         if (m & 1) e->cur = 1 - e->cur;
@@ -736,7 +782,13 @@ int run_ens_steps(slime_ensemble* e, uint32_t n) {
             int rc = ensure_lanes(e);
             if (rc != SLIME_OK) return rc;
         }
-        int rc = prepare_ens_deposits(e);
+        int rc = auto_sort(e, n);
+        if (rc != SLIME_OK) return rc;
+        if (e->sorted && !e->reorder_every) {
+            const uint64_t left = ens_sorted_steps(e) - (e->steps_done - e->sorted_since);
+            if (left < m) m = (uint32_t)left;
+        }
+        rc = prepare_ens_deposits(e);
         if (rc != SLIME_OK) return rc;
         const uint64_t kernels = lanes ? m * lane_kernels_per_step(e) : m;
         cudaGraphExec_t exec = (e->use_graphs || lanes) ? chunk_graph(e, m) : nullptr;
@@ -756,9 +808,16 @@ int run_ens_steps(slime_ensemble* e, uint32_t n) {
         after_ens_steps(e, m);
         e->launches += kernels;
         e->steps_done += m;
+        if (!e->sorted) e->unsorted_steps += m;
         n -= m;
     }
     return SLIME_OK;
+}
+
+// A colony's agents were set: in no order again.
+void unsorted(slime_ensemble* e) {
+    e->sorted = false;
+    e->unsorted_steps = 0;
 }
 
 int check_colony(slime_ensemble* e, uint32_t j) {
@@ -875,6 +934,11 @@ slime_ensemble* slime_ensemble_create(uint32_t k, const uint32_t* widths, const 
     if (rc == SLIME_OK) rc = build_agent_items(e);
     if (rc == SLIME_OK) rc = build_strip_items(e);
     if (rc == SLIME_OK) rc = size_grid(e);
+    // Untuned: the lanes for up to as many colonies as there are lanes (16 colonies
+    // of 256^2 to 1024^2, in no order: 543 us a step against 584), the one
+    // launch per step for more, whose captured chains would be that many times
+    // as many nodes.
+    if (k <= kMaxLanes) e->engine = SLIME_ENSEMBLE_LANES;
     if (rc != SLIME_OK) {
         *status = rc;
         slime_ensemble_destroy(e);
@@ -951,6 +1015,7 @@ int slime_ensemble_upload_agents(slime_ensemble* e, uint32_t j, const float* aos
     ECK(cudaMemcpyAsync(e->staging, aos, n * sizeof(float4), cudaMemcpyHostToDevice, e->stream), "uploading agents");
     AgentsSoA a = colony_soa(e, c);
     ECK(launch_aos_to_soa(e->staging, a, e->stream), "converting agents");
+    unsorted(e);
     ECK(launch_iota(a.ids, n, e->stream), "resetting agent ids");
     ECK(cudaStreamSynchronize(e->stream), "uploading agents");
     return SLIME_OK;
@@ -980,6 +1045,7 @@ int slime_ensemble_seed_agents(slime_ensemble* e, uint32_t j, uint64_t seed, flo
     ECK(launch_seed_agents(a, seed, (float)c.W, (float)c.H, hmin, hmax, c.params.agent_speed_min,
                            c.params.agent_speed_max, e->stream),
         "seeding agents");
+    unsorted(e);
     ECK(launch_iota(a.ids, c.n, e->stream), "resetting agent ids");
     ECK(cudaStreamSynchronize(e->stream), "seeding agents");
     return SLIME_OK;
@@ -988,6 +1054,7 @@ int slime_ensemble_seed_agents(slime_ensemble* e, uint32_t j, uint64_t seed, flo
 int slime_ensemble_set_reorder(slime_ensemble* e, uint32_t every, uint32_t cell_log2) {
     if (!e || cell_log2 > 15) return SLIME_ERR_INVALID_ARGUMENT;
     e->reorder_every = every;
+    unsorted(e);
     e->reorder_cell_log2 = (int)cell_log2;
     return SLIME_OK;
 }
@@ -1130,8 +1197,18 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
         cudaMemcpyAsync(s + abytes + 2 * tbytes + i * tbytes, e->counts[i], tbytes, cudaMemcpyDeviceToDevice,
                         e->stream);
     }
-    if (e->reorder_every) {
+    uint64_t agents = 0;
+    for (const Colony& c : e->colonies) agents += c.n;
+    if (e->reorder_every || (e->auto_sort && sorted_min_steps(agents) < 1000)) { // as the steps will have them
         int rrc = reorder_all(e);
+        if (rrc == SLIME_OK && !e->reorder_every) {
+            e->sorted = true;
+            e->sorted_since = e->steps_done;
+        }
+        if (rrc == SLIME_ERR_OUT_OF_MEMORY && !e->reorder_every) {
+            e->auto_sort = false;
+            rrc = SLIME_OK;
+        }
         if (rrc != SLIME_OK) {
             dev_free(snap);
             return rrc;
@@ -1141,6 +1218,10 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
     }
     const uint64_t saved_steps = e->steps_done, saved_reorder = e->reorder_every;
     e->reorder_every = 0;
+    const bool saved_auto = e->auto_sort, saved_sorted = e->sorted;
+    const uint64_t saved_unsorted = e->unsorted_steps;
+    e->auto_sort = false; // the trials' snapshot holds the slots' order as it is now
+    e->sorted = false;
     const int saved_cur = e->cur;
     const bool saved_graphs = e->use_graphs;
     e->use_graphs = false;
@@ -1241,6 +1322,9 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
     e->cur = saved_cur;
     e->use_graphs = saved_graphs;
     e->steps_done = saved_steps;
+    e->auto_sort = saved_auto;
+    e->sorted = saved_sorted;
+    e->unsorted_steps = saved_unsorted;
     e->reorder_every = saved_reorder;
     e->rows = best_rows;
     e->blocks_per_sm = best_bps;

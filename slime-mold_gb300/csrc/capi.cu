@@ -739,13 +739,19 @@ int end_sorted_run(slime_ctx* ctx) {
     return SLIME_OK;
 }
 
-// Whether the persisting-L2 window over the trail pays off for this context,
-// and on which passes: `steps` full steps (an even number) with the window on
-// both passes, on the trail pass only, on the agent pass only and without a
-// carve-out, twice each in alternation, from a snapshot of the agents and the
-// trail that is put back before every trial and at the end.  Without a
-// snapshot buffer nothing changes.
-int tune_l2_window(slime_ctx* ctx, uint32_t steps) {
+// What only whole steps show, timed on them from a snapshot of the agents and
+// the trail that is put back before every trial and at the end (without a
+// snapshot buffer nothing changes), `steps` (an even number) as the steps will
+// be run, twice each in alternation:
+//   - the trail tile, of the fastest shared-memory tile and the fastest strips
+//     (tiles[0], tiles[1]; -1 for none): strips overlap their launch with the
+//     agent pass and leave it the L1 (trail_tile.cuh), which no trial of the
+//     trail pass alone sees (512^2 with 65,536 agents: 6.5 us a step with the
+//     tile that is fastest alone, 5.4 with strips), and only in a graph;
+//   - whether the persisting-L2 window over the trail pays off, and on which
+//     passes: on both, on the trail pass only, on the agent pass only, or no
+//     carve-out.
+int tune_full_steps(slime_ctx* ctx, uint32_t steps, const int tiles[2]) {
     const size_t cells = (size_t)ctx->W * ctx->H;
     const size_t abytes = 4 * ctx->agents.n_pad * sizeof(float);
     const size_t tbytes = cells * sizeof(float);
@@ -774,37 +780,57 @@ int tune_l2_window(slime_ctx* ctx, uint32_t steps) {
         e = cudaMemcpyAsync(snap + abytes, ctx->trail[cur], tbytes, cudaMemcpyDeviceToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
-    // the window on both passes, on the trail pass only, on the agent pass
-    // only, and no carve-out at all
-    const unsigned passes[4] = {kWindowAgents | kWindowTrail, kWindowTrail, kWindowAgents, 0};
-    float total[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int round = 0; round < 2 && e == cudaSuccess; round++) {
-        for (int c = 0; c < 4 && e == cudaSuccess; c++) {
+    // `steps` steps from the snapshot, replayed from a graph where that matters
+    // (whether passes overlap); adds their time to *ms
+    auto trial = [&](float* ms, bool graph) {
+        cudaGraphExec_t exec = nullptr;
+        if (graph) invalidate_graphs(ctx);
+        if (graph && ctx->opt.use_graphs && step_graph(ctx, steps, marks, &exec) != SLIME_OK) e = cudaErrorUnknown;
+        for (int pass = 0; pass < 2 && e == cudaSuccess; pass++) { // the first warms up
+            e = restore();
+            if (e == cudaSuccess && pass) e = cudaEventRecord(e0, ctx->stream);
+            if (exec) {
+                if (e == cudaSuccess) e = cudaGraphLaunch(exec, ctx->stream);
+            } else {
+                for (uint32_t i = 0; i < (pass ? steps : 2) && e == cudaSuccess; i++) e = enqueue_step(ctx, marks, i > 0);
+            }
+            if (e == cudaSuccess && pass) e = cudaEventRecord(e1, ctx->stream);
+            ctx->launches += steps * kernels_per_step(ctx, marks);
+        }
+        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+        float t = 0.0f;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
+        *ms += t;
+    };
+    if (tiles[0] >= 0 && tiles[1] >= 0 && !ctx->opt.trail_tile) {
+        float total[2] = {0.0f, 0.0f};
+        for (int i = 0; i < 4 && e == cudaSuccess; i++) {
+            ctx->tile = tiles[i & 1];
+            trial(&total[i & 1], true);
+        }
+        if (e == cudaSuccess) ctx->tuned_tile = tiles[total[1] < total[0] ? 1 : 0];
+        choose_kernels(ctx);
+    }
+    if (ctx->opt.l2_persist && ctx->l2_persist_bytes) {
+        const unsigned passes[4] = {kWindowAgents | kWindowTrail, kWindowTrail, kWindowAgents, 0};
+        float total[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int i = 0; i < 8 && e == cudaSuccess; i++) {
+            const int c = i & 3;
             ctx->l2_tuned_off = passes[c] == 0;
             ctx->l2_window_passes = passes[c] ? passes[c] : 3;
             setup_l2(ctx);
             if (c == 0 && !ctx->l2_persist_bytes) break; // no carve-out to compare with
-            e = restore();
-            for (int w = 0; w < 2 && e == cudaSuccess; w++) e = enqueue_step(ctx, marks, w > 0);
-            if (e == cudaSuccess) e = restore();
-            if (e == cudaSuccess) e = cudaEventRecord(e0, ctx->stream);
-            for (uint32_t i = 0; i < steps && e == cudaSuccess; i++) e = enqueue_step(ctx, marks, i > 0);
-            if (e == cudaSuccess) e = cudaEventRecord(e1, ctx->stream);
-            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-            float ms = 0.0f;
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-            total[c] += ms;
-            ctx->launches += (steps + 2) * kernels_per_step(ctx, marks);
+            trial(&total[c], false);
         }
+        int best = 0;
+        const bool measured = e == cudaSuccess && total[0] > 0.0f && total[3] > 0.0f;
+        if (measured)
+            for (int c = 1; c < 4; c++)
+                if (total[c] > 0.0f && total[c] < total[best]) best = c;
+        ctx->l2_tuned_off = passes[best] == 0;
+        ctx->l2_window_passes = passes[best] ? passes[best] : 3;
+        setup_l2(ctx);
     }
-    int best = 0;
-    const bool measured = e == cudaSuccess && total[0] > 0.0f && total[3] > 0.0f;
-    if (measured)
-        for (int c = 1; c < 4; c++)
-            if (total[c] > 0.0f && total[c] < total[best]) best = c;
-    ctx->l2_tuned_off = passes[best] == 0;
-    ctx->l2_window_passes = passes[best] ? passes[best] : 3;
-    setup_l2(ctx);
     cudaError_t re = restore();
     if (re == cudaSuccess) re = cudaStreamSynchronize(ctx->stream);
     if (e0) cudaEventDestroy(e0);
@@ -812,8 +838,8 @@ int tune_l2_window(slime_ctx* ctx, uint32_t steps) {
     dev_free(snap);
     invalidate_graphs(ctx);
     ctx->last_counts_valid = false;
-    if (e != cudaSuccess) return cuda_error(ctx->err, e, "autotuning the L2 window");
-    if (re != cudaSuccess) return cuda_error(ctx->err, re, "autotuning the L2 window");
+    if (e != cudaSuccess) return cuda_error(ctx->err, e, "autotuning whole steps");
+    if (re != cudaSuccess) return cuda_error(ctx->err, re, "autotuning whole steps");
     return SLIME_OK;
 }
 
@@ -1517,6 +1543,8 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
     // Each tile runs with the deposit record the steps would use.
     float best = 1e30f;
     int best_tile = ctx->tile;
+    float best_of[2] = {1e30f, 1e30f}; // of the shared-memory tiles, of the others
+    int tile_of[2] = {-1, -1};
     const bool mk = use_marks(ctx);
     for (int t = 0; t < trail_tile_count(); t++) {
         if (!trail_tile_supported(ctx->dev, t) || (t == kTrailTileTma && !ctx->tmaps.ok)) continue;
@@ -1540,14 +1568,19 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
             best = ms;
             best_tile = t;
         }
+        const int kind = trail_tile_streams(ctx->dev, t) ? 1 : 0;
+        if (ms < best_of[kind]) {
+            best_of[kind] = ms;
+            tile_of[kind] = t;
+        }
     }
     // 2. agent-kernel shapes, on a snapshot of the agents that is put back
     // afterwards (the trial passes write agents and the deposit record).
     // With reordering on, the agents are put in Morton order first, as the
     // steps will have them.  Each shape starts from the snapshot, makes one
     // untimed pass (the copy back evicts the trail from L2) and is timed over
-    // `reps` passes in a row with the deposit record the steps will use;
-    // twice, keeping the faster.
+    // `reps` passes in a row with the deposit record the steps will use; those
+    // within a tenth of the best twice, keeping the faster.
     if (ctx->opt.reorder_every && ctx->agents.n > 0) {
         int rrc = do_reorder(ctx);
         if (rrc != SLIME_OK) return rrc;
@@ -1560,10 +1593,13 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
         if (dev_alloc((void**)&snap, abytes) == cudaSuccess) {
             CK(cudaMemcpyAsync(snap, ctx->agent_block, abytes, cudaMemcpyDeviceToDevice, ctx->stream), "snapshot");
             float best_a = 1e30f;
+            std::vector<float> first((size_t)agent_shape_count(), 0.0f);
             for (int round = 0; round < 2; round++)
                 for (int sh = 0; sh < agent_shape_count(); sh++) {
                     // without a texture the gather shapes repeat their pointer twins
                     if (agent_shape_uses_texture(sh) && !ctx->trail_tex[cur]) continue;
+                    // timed again only if it came near the best the first time
+                    if (round == 1 && first[sh] > 1.1f * best_a) continue;
                     cudaMemcpyAsync(ctx->agent_block, snap, abytes, cudaMemcpyDeviceToDevice, ctx->stream);
                     launch_agents(ctx->dev, ctx->agents, ctx->trail[cur], ctx->counts[cur], ctx->stream, sh, nullptr,
                                   ctx->trail_tex[cur], marks);
@@ -1576,6 +1612,7 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
                     float ms = 0;
                     cudaEventElapsedTime(&ms, e0, e1);
                     ctx->launches += (reps + 1) * (uint64_t)agent_pass_kernels(ctx->dev, ctx->agents.n, mk);
+                    if (round == 0) first[sh] = ms;
                     if (ms < best_a) {
                         best_a = ms;
                         best_shape = sh;
@@ -1596,12 +1633,15 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
     ctx->tuned_tile = best_tile;
     ctx->tuned_shape = best_shape;
     choose_kernels(ctx);
-    // 3. the persisting-L2 window, with the tile and shape just chosen
-    if (ctx->opt.l2_persist && ctx->agents.n > 0) {
+    // 3. the two kinds of tile and the persisting-L2 window, on whole steps
+    if (ctx->agents.n > 0) {
         ctx->l2_tuned_off = false;
         ctx->l2_window_passes = 3;
-        setup_l2(ctx);
-        if (ctx->l2_persist_bytes) return tune_l2_window(ctx, 2 * (reps < 5 ? 5 : reps));
+        if (ctx->opt.l2_persist) setup_l2(ctx);
+        // small steps: more of them
+        const uint64_t work = ctx->agents.n + cells / 4;
+        const uint32_t steps = work > 4000000 ? 4 : 2 * (reps < 5 ? 5 : reps) * (work < 400000 ? 2 : 1);
+        return tune_full_steps(ctx, steps, tile_of);
     }
     return SLIME_OK;
 }

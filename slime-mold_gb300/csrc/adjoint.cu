@@ -15,7 +15,9 @@
 // The forward is recorded with a checkpoint of agents and trail every K steps;
 // the backward replays each segment from its checkpoint (bit-identical to the
 // recorded run), keeps T_s and k_s of the segment in HBM, and runs one fused
-// stencil kernel per step backwards through it.
+// stencil kernel per step backwards through it.  The last segment, the
+// backward's first, is recorded straight into those buffers where memory
+// allows, and not replayed.
 #include <string.h>
 
 #include "ctx.h"
@@ -412,13 +414,36 @@ void drop_segment_graphs(slime_ctx* ctx) {
     ctx->adj.seg_graphs.clear();
 }
 
-void free_adjoint(slime_ctx* ctx) {
+// Gives back the buffers of the backward; the recording stays (every segment
+// can be replayed from its checkpoint).
+void release_segment(slime_ctx* ctx) {
     auto& a = ctx->adj;
+    cudaStreamSynchronize(ctx->stream);
     drop_segment_graphs(ctx);
+    for (auto it = ctx->graphs.begin(); it != ctx->graphs.end();) { // recorded segments write these buffers
+        if (it->first.second & slime_ctx::kGraphRecord) {
+            cudaGraphExecDestroy(it->second);
+            it = ctx->graphs.erase(it);
+        } else {
+            ++it;
+        }
+    }
     for (cudaTextureObject_t t : a.seg_tex)
         if (t) cudaDestroyTextureObject(t);
-    void* ptrs[] = {a.ckpt_agents, a.ckpt_ids, a.ckpt_trail, a.seg_trail, a.seg_counts, a.g[0], a.g[1],
-                    a.acc, a.agents_tmp, a.ids_tmp};
+    a.seg_tex.clear();
+    a.seg_holds = -1;
+    void** ptrs[] = {(void**)&a.seg_trail, (void**)&a.seg_counts, (void**)&a.g[0], (void**)&a.g[1],
+                     (void**)&a.acc, (void**)&a.ids_tmp, (void**)&a.agents_tmp};
+    for (void** q : ptrs) {
+        if (*q) dev_free(*q);
+        *q = nullptr;
+    }
+}
+
+void free_adjoint(slime_ctx* ctx) {
+    auto& a = ctx->adj;
+    release_segment(ctx);
+    void* ptrs[] = {a.ckpt_agents, a.ckpt_ids, a.ckpt_trail};
     for (void* q : ptrs)
         if (q) dev_free(q);
     a = slime_ctx::Adjoint();
@@ -438,6 +463,124 @@ namespace {
 // of every step 256-byte aligned, for 16-byte loads and gather textures.
 size_t segment_stride(const slime_ctx* ctx) { return ((size_t)ctx->W * ctx->H + 63) & ~(size_t)63; }
 
+size_t acc_bytes(const slime_ctx* ctx) {
+    return (4 + 3 * kSumBlocks) * sizeof(double) +
+           (size_t)adjoint_blocks(ctx->W, ctx->H) * 3 * kThreads * sizeof(float2);
+}
+
+// The buffers of the backward, as the recording's sizes have them: all of them
+// or, without memory, none.
+cudaError_t alloc_segment(slime_ctx* ctx, cudaError_t (*alloc)(slime_ctx*, void**, size_t)) {
+    auto& a = ctx->adj;
+    const size_t cells = (size_t)ctx->W * ctx->H, stride = segment_stride(ctx);
+    const uint32_t K = a.ckpt_every;
+    // W + 2 zero floats past the last trail: the sampler's discarded taps
+    const size_t trail_bytes = ((size_t)K * stride + ctx->W + 2) * sizeof(float);
+    cudaError_t e;
+    if ((e = alloc(ctx, (void**)&a.seg_trail, trail_bytes)) == cudaSuccess &&
+        (e = cudaMemsetAsync(a.seg_trail, 0, trail_bytes, ctx->stream)) == cudaSuccess &&
+        (e = alloc(ctx, (void**)&a.seg_counts, (size_t)K * stride * sizeof(uint32_t))) == cudaSuccess &&
+        (e = alloc(ctx, (void**)&a.g[0], cells * sizeof(float))) == cudaSuccess &&
+        (e = alloc(ctx, (void**)&a.g[1], cells * sizeof(float))) == cudaSuccess &&
+        (e = alloc(ctx, (void**)&a.acc, acc_bytes(ctx))) == cudaSuccess &&
+        (!a.with_ids || (e = alloc(ctx, (void**)&a.ids_tmp, a.n_pad * sizeof(uint32_t))) == cudaSuccess))
+        e = alloc(ctx, (void**)&a.agents_tmp, 4 * a.n_pad * sizeof(float));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        release_segment(ctx);
+        return e;
+    }
+    for (uint32_t i = 0; i < K && agent_shape_uses_texture(a.agent_shape); i++)
+        a.seg_tex.push_back(make_trail_texture(a.seg_trail + i * stride, ctx->W, ctx->H));
+    return cudaSuccess;
+}
+
+// m steps of `ag` from the trail in the segment's first slot, keeping T_s and
+// k_s (counts cleared by the caller); the trail after the last one goes to
+// `last`, or is not made.
+cudaError_t enqueue_forward(slime_ctx* ctx, const AgentsSoA& ag, uint32_t m, float* last) {
+    auto& a = ctx->adj;
+    const size_t stride = segment_stride(ctx);
+    const bool strips = trail_tile_streams(a.dev, a.tile);
+    cudaError_t e = cudaSuccess;
+    for (uint32_t i = 0; i < m && e == cudaSuccess; i++) {
+        float* Ti = a.seg_trail + (size_t)i * stride;
+        uint32_t* Ki = a.seg_counts + (size_t)i * stride;
+        e = launch_agents(a.dev, ag, Ti, Ki, ctx->stream, a.agent_shape, nullptr,
+                          i < a.seg_tex.size() ? a.seg_tex[i] : 0, nullptr, i > 0 && strips);
+        float* to = i + 1 < m ? Ti + stride : last;
+        if (e == cudaSuccess && to)
+            e = launch_trail(a.dev, a.tile, Ti, Ki, to, nullptr, ctx->stream, nullptr, a.n > 0);
+    }
+    return e;
+}
+
+// Whether the last segment can be recorded into the backward's buffers: they
+// are there, or are taken now from memory that is amply there (a quarter of
+// what is free; the backward would take them in any case).
+bool segment_ready(slime_ctx* ctx) {
+    auto& a = ctx->adj;
+    if (a.agents_tmp) return true;
+    size_t free_b = 0, total_b = 0;
+    const size_t bytes = ((size_t)a.ckpt_every * 2 * segment_stride(ctx) + 5 * a.n_pad) * sizeof(float);
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4) {
+        cudaGetLastError();
+        return false;
+    }
+    return alloc_segment(ctx, [](slime_ctx*, void** p, size_t b) { return dev_alloc(p, b); }) == cudaSuccess;
+}
+
+// The last m recorded steps, keeping T_s and k_s for the backward.  What they
+// leave behind is what m steps leave: the trail in the buffer that is current
+// then, the last step's counts, the agents.  The records that later steps write
+// are not touched.  Measured on 1024^2 with 1 M agents, 200 steps, segments of
+// 50: recording and backward 10.5 ms with every segment replayed, 9.5 so.
+int record_last_segment(slime_ctx* ctx, uint32_t m) {
+    auto& a = ctx->adj;
+    const size_t cells = (size_t)ctx->W * ctx->H, stride = segment_stride(ctx);
+    const int to = (m & 1) ? 1 - ctx->cur : ctx->cur;
+    CK(cudaMemcpyAsync(a.seg_trail, ctx->trail[ctx->cur], cells * sizeof(float), cudaMemcpyDeviceToDevice,
+                       ctx->stream), "keeping the trail");
+    CK(cudaMemsetAsync(a.seg_counts, 0, (size_t)m * stride * sizeof(uint32_t), ctx->stream), "clearing counts");
+    cudaGraphExec_t exec = nullptr;
+    if (ctx->opt.use_graphs) {
+        auto key = std::make_pair(m, ctx->cur | (ctx->in_sorted_run ? slime_ctx::kGraphSorted : 0) | slime_ctx::kGraphRecord);
+        auto it = ctx->graphs.find(key);
+        if (it == ctx->graphs.end()) {
+            cudaError_t ce = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
+            if (ce == cudaSuccess) ce = enqueue_forward(ctx, ctx->agents, m, ctx->trail[to]);
+            cudaGraph_t graph = nullptr;
+            cudaError_t ee = cudaStreamEndCapture(ctx->stream, &graph);
+            if (ce == cudaSuccess && ee == cudaSuccess) ee = cudaGraphInstantiate(&exec, graph, 0);
+            if (graph) cudaGraphDestroy(graph);
+            if (ce == cudaSuccess && ee == cudaSuccess) {
+                ctx->graphs[key] = exec;
+            } else {
+                cudaGetLastError();
+                exec = nullptr; // direct launches
+            }
+        } else {
+            exec = it->second;
+        }
+    }
+    if (exec)
+        CK(cudaGraphLaunch(exec, ctx->stream), "launching recorded steps");
+    else
+        CK(enqueue_forward(ctx, ctx->agents, m, ctx->trail[to]), "launching recorded steps");
+    CK(cudaMemcpyAsync(ctx->counts[1 - to], a.seg_counts + (size_t)(m - 1) * stride, cells * sizeof(uint32_t),
+                       cudaMemcpyDeviceToDevice, ctx->stream), "keeping the last step's counts");
+    ctx->launches += (uint64_t)m * (1 + agent_pass_kernels(a.dev, a.n, false));
+    ctx->steps_done += m;
+    ctx->cur = to;
+    const bool dirty[4] = {ctx->counts_dirty[0], ctx->counts_dirty[1], ctx->marks_dirty[0], ctx->marks_dirty[1]};
+    after_steps(ctx, false, m);
+    for (int i = 0; i < 2; i++) {
+        ctx->counts_dirty[i] = dirty[i] || i == 1 - to;
+        ctx->marks_dirty[i] = dirty[2 + i];
+    }
+    return SLIME_OK;
+}
+
 // The recorded steps, on the context's agents as they are now (its own, or the
 // sorted copy of begin_sorted_run).
 int record_steps(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) {
@@ -454,6 +597,7 @@ int record_steps(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) {
     if (memcmp(&a.dev, &ctx->dev, sizeof a.dev) != 0 || a.tile != ctx->tile || a.agent_shape != ctx->agent_shape)
         drop_segment_graphs(ctx);
     a.recorded = false;
+    a.seg_holds = -1;
     a.n_steps = n_steps;
     a.ckpt_every = K;
     a.n_ckpt = n_ckpt;
@@ -485,6 +629,11 @@ int record_steps(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) {
         CK(cudaMemcpyAsync(a.ckpt_trail + (size_t)j * cells, ctx->trail[ctx->cur], cells * sizeof(float),
                            cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing trail");
         uint32_t m = (n_steps - j * K) < K ? (n_steps - j * K) : K;
+        if (j + 1 == a.n_ckpt && segment_ready(ctx)) {
+            if ((rc = record_last_segment(ctx, m)) != SLIME_OK) return rc;
+            a.seg_holds = (int)j;
+            break;
+        }
         while (m > 0) {
             const bool marks = use_marks(ctx);
             if ((rc = prepare_deposits(ctx, marks)) != SLIME_OK) return rc;
@@ -537,37 +686,12 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
     cudaSetDevice(ctx->device);
     const size_t cells = (size_t)ctx->W * ctx->H;
     const uint32_t K = a.ckpt_every;
-    cudaError_t e;
     const size_t stride = segment_stride(ctx);
     const uint32_t blocks = adjoint_blocks(ctx->W, ctx->H);
-    const size_t acc_bytes = (4 + 3 * kSumBlocks) * sizeof(double) + (size_t)blocks * 3 * kThreads * sizeof(float2);
-    if (!a.agents_tmp) {
-        // W + 2 zero floats past the last trail: the sampler's discarded taps
-        const size_t trail_bytes = ((size_t)K * stride + ctx->W + 2) * sizeof(float);
-        if ((e = ctx_alloc(ctx, (void**)&a.seg_trail, trail_bytes)) == cudaSuccess &&
-            (e = cudaMemsetAsync(a.seg_trail, 0, trail_bytes, ctx->stream)) == cudaSuccess &&
-            (e = ctx_alloc(ctx, (void**)&a.seg_counts, (size_t)K * stride * sizeof(uint32_t))) == cudaSuccess &&
-            (e = ctx_alloc(ctx, (void**)&a.g[0], cells * sizeof(float))) == cudaSuccess &&
-            (e = ctx_alloc(ctx, (void**)&a.g[1], cells * sizeof(float))) == cudaSuccess &&
-            (e = ctx_alloc(ctx, (void**)&a.acc, acc_bytes)) == cudaSuccess &&
-            (!a.with_ids || (e = ctx_alloc(ctx, (void**)&a.ids_tmp, a.n_pad * sizeof(uint32_t))) == cudaSuccess))
-            e = ctx_alloc(ctx, (void**)&a.agents_tmp, 4 * a.n_pad * sizeof(float));
-        if (e != cudaSuccess) {
-            // what was allocated goes back: a later call starts anew
-            void** ptrs[] = {(void**)&a.seg_trail, (void**)&a.seg_counts, (void**)&a.g[0], (void**)&a.g[1],
-                             (void**)&a.acc, (void**)&a.ids_tmp, (void**)&a.agents_tmp};
-            for (void** q : ptrs) {
-                dev_free(*q);
-                *q = nullptr;
-            }
-            return cuda_error(ctx->err, e, "allocating adjoint buffers");
-        }
-        for (uint32_t i = 0; i < K && agent_shape_uses_texture(a.agent_shape); i++)
-            a.seg_tex.push_back(make_trail_texture(a.seg_trail + i * stride, ctx->W, ctx->H));
-    }
+    if (!a.agents_tmp) CK(alloc_segment(ctx, ctx_alloc), "allocating adjoint buffers");
     CK(cudaMemcpyAsync(a.g[0], dl_dtrail_final, cells * sizeof(float), cudaMemcpyHostToDevice, ctx->stream),
        "uploading dL/dT");
-    CK(cudaMemsetAsync(a.acc, 0, acc_bytes, ctx->stream), "clearing gradients");
+    CK(cudaMemsetAsync(a.acc, 0, acc_bytes(ctx), ctx->stream), "clearing gradients");
     double* parts = (double*)a.acc;                      // 3, then 3 x kSumBlocks, then every thread's
     float2* thread_acc = (float2*)(parts + 4 + 3 * kSumBlocks);
     int cg = 0;
@@ -579,21 +703,12 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
     tmp.ids = a.with_ids ? a.ids_tmp : nullptr;
     tmp.n = a.n;
     tmp.n_pad = a.n_pad;
-    // One segment after its restore: the replay of its m steps from the
-    // checkpoint (keeping T_s and k_s), then its m backward steps, starting
-    // from g[g0].  The same launches for every segment of m steps: captured
-    // once per (m, g0) as a CUDA graph and replayed.
-    auto enqueue_segment = [&](uint32_t m, int g0) -> cudaError_t {
-        cudaError_t ce = cudaSuccess;
-        const bool strips = trail_tile_streams(a.dev, a.tile);
-        for (uint32_t i = 0; i < m && ce == cudaSuccess; i++) {
-            float* Ti = a.seg_trail + (size_t)i * stride;
-            uint32_t* Ki = a.seg_counts + (size_t)i * stride;
-            ce = launch_agents(a.dev, tmp, Ti, Ki, ctx->stream, a.agent_shape, nullptr,
-                               i < a.seg_tex.size() ? a.seg_tex[i] : 0, nullptr, i > 0 && strips);
-            if (ce == cudaSuccess && i + 1 < m)
-                ce = launch_trail(a.dev, a.tile, Ti, Ki, Ti + stride, nullptr, ctx->stream, nullptr, a.n > 0);
-        }
+    // One segment: after its restore the replay of its m steps from the
+    // checkpoint (keeping T_s and k_s), unless they are held already, then its m
+    // backward steps, starting from g[g0].  The same launches for every segment
+    // of m steps: captured once per (m, g0, held) as a CUDA graph and replayed.
+    auto enqueue_segment = [&](uint32_t m, int g0, bool held) -> cudaError_t {
+        cudaError_t ce = held ? cudaSuccess : enqueue_forward(ctx, tmp, m, nullptr);
         int gi = g0;
         for (int64_t i = (int64_t)m - 1; i >= 0 && ce == cudaSuccess; i--) {
             // the first backward step follows the replay, the others each other
@@ -603,13 +718,13 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
         }
         return ce;
     };
-    auto segment_graph = [&](uint32_t m, int g0) -> cudaGraphExec_t {
-        auto key = std::make_pair(m, g0);
+    auto segment_graph = [&](uint32_t m, int g0, bool held) -> cudaGraphExec_t {
+        auto key = std::make_pair(m, g0 | (held ? 2 : 0));
         auto it = a.seg_graphs.find(key);
         if (it != a.seg_graphs.end()) return it->second;
         cudaGraphExec_t exec = nullptr;
         cudaError_t ce = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
-        if (ce == cudaSuccess) ce = enqueue_segment(m, g0);
+        if (ce == cudaSuccess) ce = enqueue_segment(m, g0, held);
         cudaGraph_t graph = nullptr;
         cudaError_t ee = cudaStreamEndCapture(ctx->stream, &graph);
         if (ce == cudaSuccess && ee == cudaSuccess) ee = cudaGraphInstantiate(&exec, graph, 0);
@@ -624,21 +739,25 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
     for (int64_t j = (int64_t)a.n_ckpt - 1; j >= 0; j--) {
         const uint32_t s0 = (uint32_t)j * K;
         const uint32_t m = (a.n_steps - s0) < K ? (a.n_steps - s0) : K;
-        // Replay the segment from its checkpoint, keeping T_s and k_s.
-        CK(cudaMemcpyAsync(a.agents_tmp, a.ckpt_agents + (size_t)j * 4 * a.n_pad, 4 * a.n_pad * sizeof(float),
-                           cudaMemcpyDeviceToDevice, ctx->stream), "restoring agents");
-        if (a.with_ids)
-            CK(cudaMemcpyAsync(a.ids_tmp, a.ckpt_ids + (size_t)j * a.n_pad, a.n_pad * sizeof(uint32_t),
-                               cudaMemcpyDeviceToDevice, ctx->stream), "restoring ids");
-        CK(cudaMemcpyAsync(a.seg_trail, a.ckpt_trail + (size_t)j * cells, cells * sizeof(float),
-                           cudaMemcpyDeviceToDevice, ctx->stream), "restoring trail");
-        CK(cudaMemsetAsync(a.seg_counts, 0, (size_t)m * stride * sizeof(uint32_t), ctx->stream), "clearing counts");
-        cudaGraphExec_t exec = segment_graph(m, cg);
+        const bool held = a.seg_holds == (int)j;
+        if (!held) { // replay the segment from its checkpoint, keeping T_s and k_s
+            CK(cudaMemcpyAsync(a.agents_tmp, a.ckpt_agents + (size_t)j * 4 * a.n_pad, 4 * a.n_pad * sizeof(float),
+                               cudaMemcpyDeviceToDevice, ctx->stream), "restoring agents");
+            if (a.with_ids)
+                CK(cudaMemcpyAsync(a.ids_tmp, a.ckpt_ids + (size_t)j * a.n_pad, a.n_pad * sizeof(uint32_t),
+                                   cudaMemcpyDeviceToDevice, ctx->stream), "restoring ids");
+            CK(cudaMemcpyAsync(a.seg_trail, a.ckpt_trail + (size_t)j * cells, cells * sizeof(float),
+                               cudaMemcpyDeviceToDevice, ctx->stream), "restoring trail");
+            CK(cudaMemsetAsync(a.seg_counts, 0, (size_t)m * stride * sizeof(uint32_t), ctx->stream), "clearing counts");
+            a.seg_holds = (int)j;
+        }
+        cudaGraphExec_t exec = segment_graph(m, cg, held);
         if (exec)
             CK(cudaGraphLaunch(exec, ctx->stream), "launching a backward segment");
         else
-            CK(enqueue_segment(m, cg), "replaying a segment and its backward steps");
-        ctx->launches += (uint64_t)m * agent_pass_kernels(a.dev, a.n, false) + (m - 1) + m;
+            CK(enqueue_segment(m, cg, held), "replaying a segment and its backward steps");
+        if (!held) ctx->launches += (uint64_t)m * agent_pass_kernels(a.dev, a.n, false) + (m - 1);
+        ctx->launches += m;
         if (m & 1) cg = 1 - cg;
     }
     sum_threads_kernel<<<dim3(kSumBlocks, 3), kThreads, 0, ctx->stream>>>(thread_acc, blocks, parts + 4);

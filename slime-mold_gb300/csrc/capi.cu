@@ -328,11 +328,16 @@ int valid_size(std::string& err, uint32_t W, uint32_t H, uint64_t n) {
 
 namespace slime {
 
-// Device memory for the context's other buffers.  When none is left, the copy
-// that sorted runs keep (and the sort scratch, unless the context reorders its
-// own agents) is given back first.
+// Device memory for the context's other buffers.  When none is left, the
+// backward's buffers are given back first, then the copy that sorted runs keep
+// (and the sort scratch, unless the context reorders its own agents).
 cudaError_t ctx_alloc(slime_ctx* ctx, void** p, size_t bytes) {
     cudaError_t e = dev_alloc(p, bytes);
+    if (e != cudaSuccess && ctx->adj.agents_tmp) {
+        cudaGetLastError();
+        release_segment(ctx);
+        e = dev_alloc(p, bytes);
+    }
     if (e == cudaSuccess || !ctx->sorted_block || ctx->keep_sorted) return e;
     cudaGetLastError();
     if (end_sorted_run(ctx) != SLIME_OK) return e;
@@ -560,7 +565,7 @@ int run_steps_direct(slime_ctx* ctx, uint32_t m, bool marks) {
 // The graph of m steps from the current parity with this deposit record,
 // captured on first use.
 int step_graph(slime_ctx* ctx, uint32_t m, bool marks, cudaGraphExec_t* out) {
-    auto key = std::make_pair(m, ctx->cur | (marks ? 2 : 0) | (ctx->in_sorted_run ? 4 : 0));
+    auto key = std::make_pair(m, ctx->cur | (marks ? 2 : 0) | (ctx->in_sorted_run ? slime_ctx::kGraphSorted : 0));
     auto it = ctx->graphs.find(key);
     cudaGraphExec_t exec = nullptr;
     if (it == ctx->graphs.end()) {

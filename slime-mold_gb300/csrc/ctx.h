@@ -71,7 +71,9 @@ struct slime_ctx {
     // agent pass, bit 1 the trail pass; the autotuner may keep only one)
     unsigned l2_window_passes = 3;
 
-    std::map<std::pair<uint32_t, int>, cudaGraphExec_t> graphs; // (steps, start parity | record << 1 | sorted copy << 2) -> graph
+    static constexpr int kGraphSorted = 4; // on the sorted copy
+    static constexpr int kGraphRecord = 8; // the last segment of a recording
+    std::map<std::pair<uint32_t, int>, cudaGraphExec_t> graphs; // (steps, start parity | record << 1 | the two bits below) -> graph
 
     uint64_t steps_done = 0;
     uint64_t launches = 0;
@@ -114,14 +116,15 @@ struct slime_ctx {
         float* ckpt_agents = nullptr;     // n_ckpt * 4 * n_pad floats
         uint32_t* ckpt_ids = nullptr;     // n_ckpt * n_pad (when reordered)
         float* ckpt_trail = nullptr;      // n_ckpt * cells
-        float* seg_trail = nullptr;       // T_s of the segment being replayed, one every 64-float-aligned cells
+        float* seg_trail = nullptr;       // T_s of one segment, one every 64-float-aligned cells
         uint32_t* seg_counts = nullptr;   // k_s, likewise
+        int seg_holds = -1;               // the segment whose T_s and k_s these hold
         std::vector<cudaTextureObject_t> seg_tex; // gather textures over the T_s (0 = none)
         float* g[2] = {nullptr, nullptr}; // dL/dT ping-pong
         void* acc = nullptr;              // d_decay, d_rate, d_dep, and the sums they are made from
         float* agents_tmp = nullptr;      // replay copy of the agents (4 * n_pad)
         uint32_t* ids_tmp = nullptr;
-        // captured segments (replay and backward steps) by (steps, g buffer)
+        // captured segments by (steps, g buffer | 2 where only the backward steps)
         std::map<std::pair<uint32_t, int>, cudaGraphExec_t> seg_graphs;
     } adj;
 
@@ -158,6 +161,7 @@ uint32_t sorted_min_steps(uint64_t n);
 uint32_t sorted_steps_of(const DevParams& d);
 uint32_t sorted_steps(const slime_ctx* ctx);
 int prepare_steps(slime_ctx* ctx, uint32_t n);
+void release_segment(slime_ctx* ctx);
 void free_adjoint(slime_ctx* ctx);
 void setup_l2(slime_ctx* ctx);
 constexpr unsigned kWindowAgents = 1, kWindowTrail = 2;

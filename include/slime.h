@@ -137,7 +137,8 @@ typedef struct SlimeSettings {
 typedef struct SlimeOptions {
     uint32_t use_graphs;        /* 1: capture step chunks in CUDA graphs (default 1) */
     uint32_t graph_chunk;       /* steps per captured graph (default 50) */
-    uint32_t reorder_every;     /* Morton-reorder agents every k steps, 0 = never (default 0) */
+    uint32_t reorder_every;     /* Morton-reorder agents every k steps, 0 = never (default 0): agents keep
+                                   their slots, and enough steps run on a sorted copy where memory allows */
     uint32_t reorder_cell_log2; /* Morton key granularity, log2 of a square of cells (default 2) */
     uint32_t l2_persist;        /* 1: persisting-L2 access window over the sensed trail (default 1) */
     uint32_t trail_tile;        /* 0: autotuned/default, otherwise 1 + an index into the tile table */
@@ -318,10 +319,12 @@ typedef struct SlimeGrads {
 } SlimeGrads;
 
 /* Run n_steps forward steps from the current state, keeping a checkpoint of
- * agents and trail every ckpt_every steps in device memory. */
+ * agents and trail every ckpt_every steps in device memory and, where that is
+ * amply there, the last segment's trails and counts in the buffers that
+ * slime_backward uses. */
 int slime_forward_record(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every);
 /* Back-propagate dL/dT_final (host, width*height floats) through the recorded
- * steps, recomputing each checkpoint segment; writes the parameter gradients
+ * steps, recomputing each checkpoint segment that is not kept; writes the parameter gradients
  * and, if d_trail0 is not NULL, dL/dT_0 (host, width*height floats). */
 int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* grads, float* d_trail0);
 

@@ -350,6 +350,28 @@ cudaError_t ctx_alloc(slime_ctx* ctx, void** p, size_t bytes) {
     return dev_alloc(p, bytes);
 }
 
+// Uploads a trail and finds out whether every value is finite and >= 0 (or
+// +inf), as deposit marks need it; waits for both.  *flag is a word on the
+// device, allocated on first use (without memory the host looks).
+cudaError_t upload_trail_checked(float* to, const float* trail, uint64_t n, uint32_t** flag, bool* clean,
+                                 cudaStream_t s) {
+    cudaError_t e = cudaMemcpyAsync(to, trail, n * sizeof(float), cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return e;
+    uint32_t bad = 0;
+    if (device_check_pays(n) && (*flag || dev_alloc((void**)flag, sizeof bad) == cudaSuccess)) {
+        if ((e = cudaMemsetAsync(*flag, 0, sizeof bad, s)) != cudaSuccess ||
+            (e = launch_trail_check(to, n, *flag, s)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(&bad, *flag, sizeof bad, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+            return e;
+    } else {
+        cudaGetLastError();
+        for (uint64_t i = 0; i < n; i++) bad |= !(trail[i] >= 0.0f);
+    }
+    e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) *clean = bad == 0;
+    return e;
+}
+
 void invalidate_graphs(slime_ctx* ctx) {
     for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second);
     ctx->graphs.clear();
@@ -446,9 +468,9 @@ bool keeps_trail_clean(const DevParams& d) {
 // deposition of at least 1 on a trail value t >= 0, the first deposit folds
 // t to clamp(t + dep, 0, 1) = 1 and every further one leaves it there, so the
 // fold of k deposits depends only on whether k > 0: one byte per cell carries
-// it, written with plain stores instead of 32-bit atomics, and the trail pass
-// reads 1 byte per cell instead of 4 and clears 1 instead of 4.  The result
-// is the same, bit for bit.  The host decides, from the parameters and what
+// it, set by an atomic OR on the byte's word, and the trail pass reads 1 byte
+// per cell instead of 4 and clears 1 instead of 4.  The result is the same, bit
+// for bit.  The host decides, from the parameters and what
 // it knows of the trail: clean after creation, clear and resize, checked on
 // upload, kept by steps that keep it (keeps_trail_clean).
 bool marks_allowed(const slime_ctx* ctx) {
@@ -1003,6 +1025,7 @@ void slime_destroy(slime_ctx* ctx) {
     if (ctx->staging) dev_free(ctx->staging);
     if (ctx->reorder.buf) dev_free(ctx->reorder.buf);
     if (ctx->aux) dev_free(ctx->aux);
+    if (ctx->check_flag) dev_free(ctx->check_flag);
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
     if (ctx->display_lut) dev_free(ctx->display_lut);
     if (ctx->display_image) dev_free(ctx->display_image);
@@ -1159,14 +1182,8 @@ int slime_upload_trail(slime_ctx* ctx, const float* trail, uint64_t n_cells) {
     if (n_cells != (uint64_t)ctx->W * ctx->H)
         return set_error(ctx->err, SLIME_ERR_INVALID_ARGUMENT, "trail has %llu cells, context has %llu",
                          (unsigned long long)n_cells, (unsigned long long)ctx->W * ctx->H);
-    CK(cudaMemcpyAsync(ctx->trail[ctx->cur], trail, n_cells * sizeof(float), cudaMemcpyHostToDevice, ctx->stream),
+    CK(upload_trail_checked(ctx->trail[ctx->cur], trail, n_cells, &ctx->check_flag, &ctx->trail_clean, ctx->stream),
        "uploading trail");
-    // deposit marks need every value finite and >= 0 (or +inf): checked
-    // while the copy runs
-    bool clean = true;
-    for (uint64_t i = 0; i < n_cells; i++) clean = clean && (trail[i] >= 0.0f);
-    CK(cudaStreamSynchronize(ctx->stream), "uploading trail");
-    ctx->trail_clean = clean;
     return SLIME_OK;
 }
 

@@ -81,6 +81,7 @@ struct slime_ctx {
     void* staging = nullptr; // AoS agent staging for uploads/downloads
     size_t staging_bytes = 0;
     void* aux = nullptr; // display buffer
+    uint32_t* check_flag = nullptr; // of uploaded trails
     size_t aux_bytes = 0;
     // slime_colorize_async: the LUT on the device (uploaded when it changes)
     // and the image the copy stream reads
@@ -141,6 +142,7 @@ bool keeps_trail_clean(const DevParams& d);
 bool marks_allowed(const slime_ctx* ctx);
 bool use_marks(const slime_ctx* ctx);
 int prepare_deposits(slime_ctx* ctx, bool marks);
+cudaError_t upload_trail_checked(float* to, const float* trail, uint64_t n, uint32_t** flag, bool* clean, cudaStream_t s);
 cudaError_t enqueue_step(slime_ctx* ctx, bool marks, bool chained);
 void after_steps(slime_ctx* ctx, bool marks, uint32_t m);
 uint64_t kernels_per_step(const slime_ctx* ctx, bool marks);

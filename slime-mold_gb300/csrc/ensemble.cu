@@ -276,6 +276,7 @@ struct slime_ensemble {
     uint64_t total_slots = 0, total_cells = 0;
     float* agent_block = nullptr; // x | y | angle | speed, total_slots each
     uint32_t* ids = nullptr;      // slot -> colony-local agent id (identity until reordered)
+    uint32_t* check_flag = nullptr; // of uploaded trails
     uint32_t reorder_every = 0;
     int reorder_cell_log2 = 2;
     uint64_t steps_done = 0;
@@ -958,7 +959,7 @@ void slime_ensemble_destroy(slime_ensemble* e) {
         for (int i = 0; i < 2; i++)
             if (c.tex[i]) cudaDestroyTextureObject(c.tex[i]);
     void* ptrs[] = {e->agent_block, e->ids, e->trail[0], e->trail[1], e->counts[0], e->counts[1], e->marks[0],
-                    e->marks[1], e->d_cols, e->d_agent_items, e->d_strip_items, e->d_bar, e->staging,
+                    e->marks[1], e->d_cols, e->check_flag, e->d_agent_items, e->d_strip_items, e->d_bar, e->staging,
                     e->reorder.buf, e->lane_reorder[0].buf, e->lane_reorder[1].buf, e->lane_reorder[2].buf};
     for (void* p : ptrs)
         if (p) dev_free(p);
@@ -1064,14 +1065,8 @@ int slime_ensemble_upload_trail(slime_ensemble* e, uint32_t j, const float* trai
     if (rc != SLIME_OK) return rc;
     Colony& c = e->colonies[j];
     if (!trail || n_cells != (uint64_t)c.W * c.H) return ens_fail(e, SLIME_ERR_INVALID_ARGUMENT, "trail size mismatch");
-    ECK(cudaMemcpyAsync(e->trail[e->cur] + c.trail_off, trail, n_cells * sizeof(float), cudaMemcpyHostToDevice,
-                        e->stream), "uploading trail");
-    // deposit marks need every value finite and >= 0 (or +inf): checked
-    // while the copy runs
-    bool clean = true;
-    for (uint64_t i = 0; i < n_cells; i++) clean = clean && (trail[i] >= 0.0f);
-    ECK(cudaStreamSynchronize(e->stream), "uploading trail");
-    c.trail_clean = clean;
+    ECK(upload_trail_checked(e->trail[e->cur] + c.trail_off, trail, n_cells, &e->check_flag, &c.trail_clean, e->stream),
+        "uploading trail");
     return SLIME_OK;
 }
 

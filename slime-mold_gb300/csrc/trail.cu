@@ -51,6 +51,15 @@ cudaError_t launch_stream_rows(const DevParams& p, const float* in, const D* cin
     return launch_stream<2, true, ROWS, D>(p, in, cin, out, cz, s, win, pdl);
 }
 
+// Sets *flag where a value is negative or NaN.
+__global__ void trail_check_kernel(const float* __restrict__ t, uint64_t n, uint32_t* __restrict__ flag) {
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    bool bad = false;
+#pragma unroll 4
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) bad |= !(__ldg(t + i) >= 0.0f);
+    if (bad) *flag = 1;
+}
+
 const TrailTile kTiles[] = {{64, 8}, {64, 16}, {64, 32}, {128, 8}, {128, 16}, {128, 32}, {128, 64}};
 constexpr int kNumTiles = (int)(sizeof(kTiles) / sizeof(kTiles[0]));
 
@@ -110,6 +119,19 @@ bool trail_tile_supported(const DevParams& p, int tile) {
 }
 
 bool trail_tile_streams(const DevParams& p, int tile) { return tile >= kNumTiles && trail_tile_supported(p, tile); }
+
+// Whether the values of an uploaded trail are looked at on the device, where
+// they just arrived, or by the host (which deposit marks want finite and >= 0,
+// or +inf).  An upload takes, host (scalar loop, the only one before; an OR
+// over all values, which vectorises, takes 10 us less at 256^2) / device: 128^2
+// 15.5 / 28.7 us, 256^2 40.9 / 30.3, 512^2 117 / 35, 1024^2 431 / 53, 4096^2
+// 6689 / 423 (of which the copy takes all but 20).
+bool device_check_pays(uint64_t cells) { return cells >= 65536; }
+cudaError_t launch_trail_check(const float* t, uint64_t n, uint32_t* flag, cudaStream_t s) {
+    const uint64_t blocks = (n + 1023) / 1024;
+    trail_check_kernel<<<(unsigned)(blocks < 1216 ? blocks : 1216), 256, 0, s>>>(t, n, flag);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_trail_marks(const DevParams& p, int tile, const float* in, const uint8_t* marks_in, float* out,
                                uint8_t* marks_zero, cudaStream_t s, const cudaAccessPolicyWindow* win, bool pdl,

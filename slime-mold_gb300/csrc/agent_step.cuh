@@ -30,6 +30,7 @@ namespace slime {
 // in the grid, and NaN fails both compares), on trails at least 2 wide and
 // high, the only ones that have a texture.
 struct TrailPtr {
+    static constexpr bool kJitter = true;
     const float* __restrict__ t;
     struct Tap {
         float v00, v10, v01, v11, dx, dy;
@@ -62,6 +63,7 @@ struct TrailPtr {
     }
 };
 struct TrailTex {
+    static constexpr bool kJitter = true;
     cudaTextureObject_t t;
     struct Tap {
         float4 g;
@@ -95,6 +97,23 @@ struct TrailTex {
     }
 };
 
+// A reader for launches without jitter (the default settings' 0, and half of the
+// presets'): there the hash r only enters the heading as (2r - 1) * 0, a zero.
+// Adding one changes nothing but the sign of a heading of -0, and the hash is
+// finite where the position is far from overflowing it: else any r does, and
+// the hash is not worked out (jitter_matters).  A variant of the kernels and
+// not a branch on p.jitter: that branch costs the launches with jitter 1 us of
+// 203 (4096^2).  For the texture shapes only, pairs of agents bound by
+// instruction issue: with / without the hash 203 / 191 us at 4096^2, a step of
+// 10 M agents on 1600x900 128 / 122, of 1 M on 1024^2 18.9 / 18.0.  One agent per
+// thread hides the hash behind its loads: 1001x777 15.1 / 15.0 us a step,
+// caller-owned agents on 3001x2003 162.0 / 163.9.
+template <class Trail>
+struct NoJitter : Trail {
+    static constexpr bool kJitter = false;
+    __device__ __host__ __forceinline__ NoJitter(const Trail& t) : Trail(t) {}
+};
+
 // The three sensor footprints of an agent (compute.wgsl:75-95), fetched.
 template <class Trail>
 struct Senses {
@@ -117,6 +136,15 @@ __device__ __forceinline__ Senses<Trail> agent_sense(const DevParams& p, float x
     s.right = trail.fetch(p, slm_add(x, slm_mul(p.sensor_dist, cr)), slm_add(y, slm_mul(p.sensor_dist, sr)));
     s.center = trail.fetch(p, slm_add(x, slm_mul(p.sensor_dist, cc)), slm_add(y, slm_mul(p.sensor_dist, sc)));
     return s;
+}
+
+// Without jitter: whether the hash of an agent decides something all the same.
+__device__ __forceinline__ bool jitter_matters(float x, float y, float angle) {
+    return !(slm_add(slm_abs(x), slm_abs(y)) < 1e30f) || slm_f2u_bits(angle) == 0x80000000u;
+}
+static __device__ __noinline__ float jitter_hash_cold(int32_t i, float x, float y) { return slm_jitter_hash(i, x, y); }
+static __device__ __noinline__ float2 jitter_hash2_cold(int32_t ia, float xa, float ya, int32_t ib, float xb, float yb) {
+    return make_float2(slm_jitter_hash(ia, xa, ya), slm_jitter_hash(ib, xb, yb));
 }
 
 // compute.wgsl:72 and 98-122: the speed clamp, the turn from the sensor
@@ -173,7 +201,9 @@ __device__ __forceinline__ int agent_step(const DevParams& p, float& x, float& y
                                           int32_t index, const Trail& trail) {
     const Senses<Trail> s = agent_sense(p, x, y, angle, trail);
     // the hash needs no sample: it is worked out while the footprints load
-    const float rv = slm_jitter_hash(index, x, y);
+    float rv = 0.0f;
+    if (Trail::kJitter) rv = slm_jitter_hash(index, x, y);
+    else if (jitter_matters(x, y, angle)) rv = jitter_hash_cold(index, x, y);
     return agent_finish(p, x, y, angle, speed, rv, Trail::value(s.left), Trail::value(s.right),
                         Trail::value(s.center));
 }
@@ -251,8 +281,13 @@ __device__ __forceinline__ void agent_step2(const DevParams& p, float& xa, float
     const float2 mcb = __fmul2_rn(make_float2(d, d), make_float2(ccb, scb));
     const typename Trail::Tap cb = trail.fetch(p, slm_add(xb, mcb.x), slm_add(yb, mcb.y));
     // the hashes need no sample: worked out while the footprints load
-    float rva, rvb;
-    slm_jitter_hash2(ia, xa, ya, ib, xb, yb, &rva, &rvb);
+    float rva = 0.0f, rvb = 0.0f;
+    if (Trail::kJitter) {
+        slm_jitter_hash2(ia, xa, ya, ib, xb, yb, &rva, &rvb);
+    } else if (jitter_matters(xa, ya, tha) || jitter_matters(xb, yb, thb)) {
+        const float2 r = jitter_hash2_cold(ia, xa, ya, ib, xb, yb);
+        rva = r.x, rvb = r.y;
+    }
     agent_turn(p, tha, va, rva, Trail::value(la), Trail::value(ra), Trail::value(ca));
     agent_turn(p, thb, vb, rvb, Trail::value(lb), Trail::value(rb), Trail::value(cb));
     // the new headings are wrapped into [0, 2pi] (or NaN, whose sin and cos

@@ -442,6 +442,22 @@ int agent_pass_kernels(const DevParams& p, uint64_t n, bool marks) {
     return wy > 1 ? 2 : 1; // some agent is visited twice only with two or more rows
 }
 
+namespace {
+
+// The kernel of a shape that samples the texture.
+template <class Tex>
+cudaError_t launch_texture_shape(const DevParams& p, const AgentsSoA& a, const Tex& tt, uint32_t* counts, cudaStream_t s,
+                                 int shape, const cudaAccessPolicyWindow* win, uint8_t* marks, bool pdl) {
+    switch (shape) {
+    case 12: return launch_agents_variant<2, 256, 0>(p, a, tt, counts, marks, s, win, pdl);
+    case 13: return launch_agents_persistent<2, 256, 0>(p, a, tt, counts, marks, s, win, pdl);
+    case 15: return launch_agents_persistent<2, 256, 4>(p, a, tt, counts, marks, s, win, pdl);
+    default: return launch_agents_persistent<2, 128, 0>(p, a, tt, counts, marks, s, win, pdl);
+    }
+}
+
+} // namespace
+
 cudaError_t launch_agents(const DevParams& p, const AgentsSoA& a, const float* trail, uint32_t* counts,
                           cudaStream_t s, int shape, const cudaAccessPolicyWindow* win, cudaTextureObject_t tex,
                           uint8_t* marks, bool pdl) {
@@ -459,16 +475,12 @@ cudaError_t launch_agents(const DevParams& p, const AgentsSoA& a, const float* t
                                                                           span, counts);
         return cudaGetLastError();
     }
-    const TrailPtr tp{trail};
     if (agent_shape_uses_texture(shape) && tex) {
         const TrailTex tt{tex};
-        switch (shape) {
-        case 12: return launch_agents_variant<2, 256, 0>(p, a, tt, counts, marks, s, win, pdl);
-        case 13: return launch_agents_persistent<2, 256, 0>(p, a, tt, counts, marks, s, win, pdl);
-        case 15: return launch_agents_persistent<2, 256, 4>(p, a, tt, counts, marks, s, win, pdl);
-        default: return launch_agents_persistent<2, 128, 0>(p, a, tt, counts, marks, s, win, pdl);
-        }
+        if (p.jitter == 0.0f) return launch_texture_shape(p, a, NoJitter<TrailTex>(tt), counts, s, shape, win, marks, pdl);
+        return launch_texture_shape(p, a, tt, counts, s, shape, win, marks, pdl);
     }
+    const TrailPtr tp{trail};
     switch (shape) {
     case 1:
     case 12: return launch_agents_variant<2, 256, 0>(p, a, tp, counts, marks, s, win, pdl);

@@ -610,6 +610,14 @@ uint32_t ens_sorted_steps(const slime_ensemble* e) {
     return steps;
 }
 
+// No scratch memory for a sort: the steps go on in the slots' order as it is,
+// without another sort to run up to.
+void give_up_auto_sort(slime_ensemble* e) {
+    e->auto_sort = false;
+    e->sorted = false;
+    e->err.clear();
+}
+
 // Before n steps: sort the colonies where that pays (the bounds of a single
 // context's copy, on the agents of all): 16 colonies of 256^2 to 1024^2 take 258
 // us a step sorted and 543 in no order.  Without scratch memory it is given up.
@@ -622,8 +630,7 @@ int auto_sort(slime_ensemble* e, uint32_t n) {
     if (!due) return SLIME_OK;
     const int rc = reorder_all(e);
     if (rc == SLIME_ERR_OUT_OF_MEMORY) {
-        e->auto_sort = false;
-        e->err.clear();
+        give_up_auto_sort(e);
         return SLIME_OK;
     }
     e->sorted = rc == SLIME_OK;
@@ -753,7 +760,7 @@ int prepare_ens_steps(slime_ensemble* e, uint32_t n) {
         if (e->reorder_every) {
             uint64_t to_next = e->reorder_every - steps % e->reorder_every;
             if (to_next < m) m = (uint32_t)to_next;
-        } else if (e->sorted || e->unsorted_steps + n >= sorted_min_steps(agents)) {
+        } else if (e->auto_sort && (e->sorted || e->unsorted_steps + n >= sorted_min_steps(agents))) {
             if (age >= aged) age = 0;
             if (aged - age < m) m = aged - age;
             age += m;
@@ -785,7 +792,7 @@ int run_ens_steps(slime_ensemble* e, uint32_t n) {
         }
         int rc = auto_sort(e, n);
         if (rc != SLIME_OK) return rc;
-        if (e->sorted && !e->reorder_every) {
+        if (e->sorted && e->auto_sort && !e->reorder_every) {
             const uint64_t left = ens_sorted_steps(e) - (e->steps_done - e->sorted_since);
             if (left < m) m = (uint32_t)left;
         }
@@ -1201,7 +1208,7 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
             e->sorted_since = e->steps_done;
         }
         if (rrc == SLIME_ERR_OUT_OF_MEMORY && !e->reorder_every) {
-            e->auto_sort = false;
+            give_up_auto_sort(e);
             rrc = SLIME_OK;
         }
         if (rrc != SLIME_OK) {

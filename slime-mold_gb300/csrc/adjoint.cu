@@ -551,7 +551,7 @@ int record_last_segment(slime_ctx* ctx, uint32_t m) {
             if (ce == cudaSuccess) ce = enqueue_forward(ctx, ctx->agents, m, ctx->trail[to]);
             cudaGraph_t graph = nullptr;
             cudaError_t ee = cudaStreamEndCapture(ctx->stream, &graph);
-            if (ce == cudaSuccess && ee == cudaSuccess) ee = cudaGraphInstantiate(&exec, graph, 0);
+            if (ce == cudaSuccess && ee == cudaSuccess) ee = instantiate_graph(&exec, graph);
             if (graph) cudaGraphDestroy(graph);
             if (ce == cudaSuccess && ee == cudaSuccess) {
                 ctx->graphs[key] = exec;
@@ -639,7 +639,14 @@ int record_steps(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) {
             if ((rc = prepare_deposits(ctx, marks)) != SLIME_OK) return rc;
             const uint32_t chunk = ctx->opt.graph_chunk ? ctx->opt.graph_chunk : 50;
             const uint32_t take = m < chunk ? m : chunk;
-            rc = ctx->opt.use_graphs ? run_steps_graph(ctx, take, marks) : run_steps_direct(ctx, take, marks);
+            // a graph that cannot be made must not end a recording that is under way
+            cudaGraphExec_t exec = nullptr;
+            const bool graph = ctx->opt.use_graphs && step_graph(ctx, take, marks, &exec) == SLIME_OK;
+            if (!graph) {
+                cudaGetLastError();
+                ctx->err.clear();
+            }
+            rc = graph ? run_steps_graph(ctx, take, marks) : run_steps_direct(ctx, take, marks);
             if (rc != SLIME_OK) return rc;
             after_steps(ctx, marks, take);
             m -= take;
@@ -662,10 +669,11 @@ int slime_forward_record(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) 
     if (rc != SLIME_OK) return rc;
     if ((rc = begin_sorted_run(ctx, n_steps)) != SLIME_OK) return rc;
     ctx->keep_sorted = ctx->in_sorted_run;
+    const uint64_t before = ctx->steps_done;
     rc = record_steps(ctx, n_steps, ckpt_every);
     ctx->keep_sorted = false;
-    if (rc == SLIME_ERR_OUT_OF_MEMORY && ctx->in_sorted_run) {
-        // no step was made: on the context's own agents, without the copy
+    if (rc == SLIME_ERR_OUT_OF_MEMORY && ctx->in_sorted_run && ctx->steps_done == before) {
+        // before the first step: on the context's own agents, without the copy
         if ((rc = end_sorted_run(ctx)) != SLIME_OK) return rc;
         release_sorted(ctx);
         ctx->sorted_refused = true;
@@ -727,7 +735,7 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
         if (ce == cudaSuccess) ce = enqueue_segment(m, g0, held);
         cudaGraph_t graph = nullptr;
         cudaError_t ee = cudaStreamEndCapture(ctx->stream, &graph);
-        if (ce == cudaSuccess && ee == cudaSuccess) ee = cudaGraphInstantiate(&exec, graph, 0);
+        if (ce == cudaSuccess && ee == cudaSuccess) ee = instantiate_graph(&exec, graph);
         if (graph) cudaGraphDestroy(graph);
         if (ce != cudaSuccess || ee != cudaSuccess) {
             cudaGetLastError();

@@ -19,6 +19,7 @@
 
 #include <stdlib.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <string>
@@ -144,6 +145,16 @@ void dev_free(void* p) {
         }
     }
     cudaFree(p);
+}
+
+cudaError_t instantiate_graph(cudaGraphExec_t* exec, cudaGraph_t graph) {
+    static const uint64_t failing = [] {
+        const char* v = getenv("SLIME_FAIL_GRAPH");
+        return (v && *v) ? (uint64_t)strtoull(v, nullptr, 10) : (uint64_t)0;
+    }();
+    static std::atomic<uint64_t> made{0};
+    if (failing && ++made == failing) return cudaErrorMemoryAllocation;
+    return cudaGraphInstantiate(exec, graph, 0);
 }
 
 int set_error(std::string& err, int code, const char* fmt, ...) {
@@ -603,7 +614,7 @@ int step_graph(slime_ctx* ctx, uint32_t m, bool marks, cudaGraphExec_t* out) {
             return cuda_error(ctx->err, ce, "capturing steps");
         }
         CK(ee, "ending graph capture");
-        cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
+        cudaError_t ie = instantiate_graph(&exec, graph);
         cudaGraphDestroy(graph);
         CK(ie, "instantiating step graph");
         ctx->graphs[key] = exec;

@@ -90,6 +90,10 @@ cudaError_t launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cu
 // the out-of-memory paths be tested without exhausting a real GPU.
 cudaError_t dev_alloc(void** p, size_t bytes);
 void dev_free(void* p);
+// Step graphs are instantiated through this function.  When the environment
+// variable SLIME_FAIL_GRAPH holds a number k, the process's k-th one fails with
+// cudaErrorMemoryAllocation: the same for graphs that find no memory.
+cudaError_t instantiate_graph(cudaGraphExec_t* exec, cudaGraph_t graph);
 
 // Translate SlimeParams into DevParams; returns false (with a message) on
 // values the kernels cannot honour.

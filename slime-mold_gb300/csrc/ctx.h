@@ -150,6 +150,7 @@ uint64_t kernels_per_step(const slime_ctx* ctx, bool marks);
 // the agents it updates first.
 int ensure_dispatch_order(slime_ctx* ctx);
 int run_steps(slime_ctx* ctx, uint32_t n);
+int step_graph(slime_ctx* ctx, uint32_t m, bool marks, cudaGraphExec_t* out);
 int run_steps_direct(slime_ctx* ctx, uint32_t m, bool marks);
 int run_steps_graph(slime_ctx* ctx, uint32_t m, bool marks);
 int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps);

@@ -726,7 +726,7 @@ cudaGraphExec_t chunk_graph(slime_ensemble* e, uint32_t m) {
     cudaGraph_t g = nullptr;
     cudaError_t ee = cudaStreamEndCapture(e->stream, &g);
     e->cur = saved;
-    if (ce == cudaSuccess && ee == cudaSuccess) ee = cudaGraphInstantiate(&exec, g, 0);
+    if (ce == cudaSuccess && ee == cudaSuccess) ee = instantiate_graph(&exec, g);
     if (g) cudaGraphDestroy(g);
     if (ce != cudaSuccess || ee != cudaSuccess) {
         cudaGetLastError();

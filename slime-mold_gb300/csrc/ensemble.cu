@@ -559,8 +559,12 @@ cudaError_t enqueue_lane_steps(slime_ensemble* e, uint32_t m) {
 // its colony-local id).  With the lanes engine's lanes in place the colonies'
 // sorts run on four of them at once (largest first, each onto the lane with
 // the fewest agents so far), each of those lanes with its own sort scratch;
-// otherwise one after another on the ensemble's stream.
-int reorder_all(slime_ensemble* e) {
+// otherwise one after another on the ensemble's stream.  With `fitting` only
+// the colonies that launch_reorder takes.
+int reorder_all(slime_ensemble* e, bool fitting = false) {
+    auto sorts = [&](const Colony& c) {
+        return c.n > 0 && (!fitting || reorder_fits(c.W, c.H, e->reorder_cell_log2));
+    };
     const size_t nr = e->lanes.size() < 4 ? e->lanes.size() : 4;
     cudaError_t ce = cudaSuccess;
     if (e->engine == SLIME_ENSEMBLE_LANES && nr > 1) {
@@ -568,7 +572,7 @@ int reorder_all(slime_ensemble* e) {
         for (size_t l = 0; l < nr; l++) ECK(cudaStreamWaitEvent(e->lanes[l], e->fork_ev, 0), "forking reorders");
         std::vector<uint32_t> order;
         for (uint32_t j = 0; j < (uint32_t)e->colonies.size(); j++)
-            if (e->colonies[j].n) order.push_back(j);
+            if (sorts(e->colonies[j])) order.push_back(j);
         std::stable_sort(order.begin(), order.end(),
                          [&](uint32_t a, uint32_t b) { return e->colonies[a].n > e->colonies[b].n; });
         std::vector<uint64_t> load(nr, 0);
@@ -590,7 +594,7 @@ int reorder_all(slime_ensemble* e) {
         }
     } else {
         for (const Colony& c : e->colonies) {
-            if (c.n == 0 || ce != cudaSuccess) continue;
+            if (!sorts(c) || ce != cudaSuccess) continue;
             AgentsSoA a = colony_soa(e, c);
             ce = launch_reorder(a, a, c.W, c.H, e->reorder_cell_log2, e->reorder, e->stream);
             e->launches += kReorderKernels;
@@ -599,6 +603,14 @@ int reorder_all(slime_ensemble* e) {
     ECK(ce, "reordering agents");
     e->last_reorder_step = e->steps_done;
     return SLIME_OK;
+}
+
+// The agents of the colonies that can be sorted.
+uint64_t sortable_agents(const slime_ensemble* e) {
+    uint64_t n = 0;
+    for (const Colony& c : e->colonies)
+        if (reorder_fits(c.W, c.H, e->reorder_cell_log2)) n += c.n;
+    return n;
 }
 
 // Steps after which the colonies are sorted again when no schedule says so: when
@@ -619,16 +631,14 @@ void give_up_auto_sort(slime_ensemble* e) {
 }
 
 // Before n steps: sort the colonies where that pays (the bounds of a single
-// context's copy, on the agents of all): 16 colonies of 256^2 to 1024^2 take 258
+// context's copy, on the agents of all that can be sorted): 16 colonies of 256^2 to 1024^2 take 258
 // us a step sorted and 543 in no order.  Without scratch memory it is given up.
 int auto_sort(slime_ensemble* e, uint32_t n) {
     if (e->reorder_every || !e->auto_sort) return SLIME_OK;
-    uint64_t agents = 0;
-    for (const Colony& c : e->colonies) agents += c.n;
     const bool due = e->sorted ? e->steps_done - e->sorted_since >= ens_sorted_steps(e)
-                               : (uint64_t)n + e->unsorted_steps >= sorted_min_steps(agents);
+                               : (uint64_t)n + e->unsorted_steps >= sorted_min_steps(sortable_agents(e));
     if (!due) return SLIME_OK;
-    const int rc = reorder_all(e);
+    const int rc = reorder_all(e, true);
     if (rc == SLIME_ERR_OUT_OF_MEMORY) {
         give_up_auto_sort(e);
         return SLIME_OK;
@@ -751,8 +761,8 @@ int prepare_ens_steps(slime_ensemble* e, uint32_t n) {
     int rc = prepare_ens_deposits(e);
     if (rc != SLIME_OK) return rc;
     const int saved = e->cur;
-    uint64_t steps = e->steps_done, agents = 0;
-    for (const Colony& c : e->colonies) agents += c.n;
+    uint64_t steps = e->steps_done;
+    const uint64_t agents = sortable_agents(e);
     const uint32_t aged = ens_sorted_steps(e);
     uint32_t age = e->sorted ? (uint32_t)(e->steps_done - e->sorted_since) : 0u;
     while (n > 0) {
@@ -1199,10 +1209,8 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
         cudaMemcpyAsync(s + abytes + 2 * tbytes + i * tbytes, e->counts[i], tbytes, cudaMemcpyDeviceToDevice,
                         e->stream);
     }
-    uint64_t agents = 0;
-    for (const Colony& c : e->colonies) agents += c.n;
-    if (e->reorder_every || (e->auto_sort && sorted_min_steps(agents) < 1000)) { // as the steps will have them
-        int rrc = reorder_all(e);
+    if (e->reorder_every || (e->auto_sort && sorted_min_steps(sortable_agents(e)) < 1000)) { // as the steps will have them
+        int rrc = reorder_all(e, !e->reorder_every);
         if (rrc == SLIME_OK && !e->reorder_every) {
             e->sorted = true;
             e->sorted_since = e->steps_done;

@@ -149,6 +149,8 @@ struct ReorderScratch {
     size_t bytes = 0;
 };
 cudaError_t launch_iota(uint32_t* ids, uint64_t n, cudaStream_t s);
+// Whether a W x H trail has a Morton key of 32 bits (else launch_reorder refuses).
+bool reorder_fits(uint32_t W, uint32_t H, int cell_log2);
 // The agents of `a` into `to` in Morton order (`to` may be `a` itself, with an id
 // array; without ids a's slots are the ids); agents with id >= `visited` go to
 // the last slots.  Six kernels.

@@ -178,17 +178,31 @@ cudaError_t launch_iota(uint32_t* ids, uint64_t n, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+namespace {
+
+// Bits of the Morton key per side.
+int key_bits(uint32_t W, uint32_t H, int cell_log2) {
+    const uint32_t dx = (W + (1u << cell_log2) - 1) >> cell_log2;
+    const uint32_t dy = (H + (1u << cell_log2) - 1) >> cell_log2;
+    const uint32_t d = dx > dy ? dx : dy;
+    int L = 0;
+    while ((1u << L) < d) L++;
+    return L;
+}
+
+} // namespace
+
+bool reorder_fits(uint32_t W, uint32_t H, int cell_log2) {
+    return key_bits(W, H, cell_log2) <= 16;
+}
+
 cudaError_t launch_reorder(const AgentsSoA& a, const AgentsSoA& to, uint32_t W, uint32_t H, int cell_log2,
                            ReorderScratch& scratch, cudaStream_t s, uint64_t visited) {
     if (a.n == 0) return cudaSuccess;
     if (!to.ids) return cudaErrorInvalidValue;
     if (cell_log2 < 0) cell_log2 = 0;
     if (cell_log2 > 15) cell_log2 = 15;
-    uint32_t dx = (W + (1u << cell_log2) - 1) >> cell_log2;
-    uint32_t dy = (H + (1u << cell_log2) - 1) >> cell_log2;
-    uint32_t d = dx > dy ? dx : dy;
-    int L = 0;
-    while ((1u << L) < d) L++;
+    const int L = key_bits(W, H, cell_log2);
     if (L > 16) return cudaErrorInvalidValue;
     const bool partition = visited < a.n;
     if (partition && L > 15) return cudaErrorInvalidValue; // no key left past the Morton codes

@@ -75,3 +75,35 @@ np.savez({str(path)!r}, **{{f"a{{j}}": ens.download_agents(j) for j in range(K)}
             sim.step(120)
             assert_bitexact(got[f"a{j}"], sim.download_agents(), f"agents of {j}")
             assert_bitexact(got[f"t{j}"], sim.download_trail(), f"trail of {j}")
+
+
+@pytest.mark.parametrize("engine", [0, 1])
+@pytest.mark.parametrize("tuned", [False, True])
+def test_colonies_too_wide_to_sort_step(gpu, engine, tuned):
+    """A side of more than 262,144 cells has no sort key: such a colony steps as
+    its agents come, the others of the ensemble are sorted.  By a schedule it
+    is still refused."""
+    import slime_gb300 as sg
+    sizes = [(262_148, 8, 40_000), (128, 96, 30_000)]
+    params = [config0_params(W, H, agent_speed_min=60.0, agent_speed_max=125.0) for W, H, _ in sizes]
+    ens = sg.Ensemble([s[0] for s in sizes], [s[1] for s in sizes], [s[2] for s in sizes], params)
+    ens.set_engine(engine)
+    sims = [sg.Simulation(W, H, n, p) for (W, H, n), p in zip(sizes, params)]
+    for j, (W, H, n) in enumerate(sizes):
+        agents = agents_uniform(n, W, H, 60.0, 125.0, seed=j)
+        ens.upload_agents(j, agents)
+        sims[j].upload_agents(agents)
+    if tuned:
+        ens.autotune(1)
+        ens.set_engine(engine)
+    ens.prepare_steps(70)
+    for k in (70, 20):
+        ens.step(k)
+    for j, sim in enumerate(sims):
+        for _ in range(90):
+            sim.step(1)
+        assert_bitexact(ens.download_agents(j), sim.download_agents(), f"agents of {j}")
+        assert_bitexact(ens.download_trail(j), sim.download_trail(), f"trail of {j}")
+    ens.set_reorder(5, 2)
+    with pytest.raises(sg.SlimeError):
+        ens.step(5)

@@ -698,8 +698,10 @@ void release_sorted(slime_ctx* ctx) {
     ctx->sorted_block = nullptr;
 }
 
-// Whether n_steps are run on a copy; allocates it on first use, only from
-// memory that is amply there (a quarter of what is free, and 4 GiB at most).
+// Whether n_steps are run on a copy; allocates it on first use, only where it and
+// the sort's scratch (44 bytes an agent and 4 a sort key, see reorder.cu) come
+// from memory that is amply there: a quarter of what is free, and 4 GiB at most
+// for the copy.
 bool sorted_run_ready(slime_ctx* ctx, uint32_t n_steps) {
     const uint64_t n = ctx->agents.n, n_pad = ctx->agents.n_pad;
     if (ctx->opt.reorder_every || ctx->agents.ids || ctx->sorted_refused ||
@@ -708,8 +710,10 @@ bool sorted_run_ready(slime_ctx* ctx, uint32_t n_steps) {
         return false;
     if (!ctx->sorted_block) {
         const size_t bytes = 5 * n_pad * sizeof(float);
+        const size_t scratch = reorder_scratch_bytes(n, ctx->W, ctx->H, 2);
         size_t free_b = 0, total_b = 0;
-        if (bytes > (4ull << 30) || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 3 * bytes > free_b / 4 ||
+        if (!scratch || bytes > (4ull << 30) || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess ||
+            bytes + (ctx->reorder.bytes < scratch ? scratch : 0) > free_b / 4 ||
             dev_alloc(&ctx->sorted_block, bytes) != cudaSuccess) {
             cudaGetLastError();
             ctx->sorted_block = nullptr;
@@ -733,7 +737,7 @@ int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps) {
     to.v = to.th + to.n_pad;
     to.ids = (uint32_t*)(to.v + to.n_pad);
     const cudaError_t e = launch_reorder(ctx->agents, to, ctx->W, ctx->H, 2, ctx->reorder, ctx->stream);
-    if (e == cudaErrorMemoryAllocation || e == cudaErrorInvalidValue) { // no sort scratch, or no Morton code this wide
+    if (e == cudaErrorMemoryAllocation) { // no sort scratch
         cudaGetLastError();
         ctx->sorted_refused = true;
         release_sorted(ctx);

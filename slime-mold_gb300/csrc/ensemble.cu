@@ -28,6 +28,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -555,15 +556,19 @@ cudaError_t enqueue_lane_steps(slime_ensemble* e, uint32_t m) {
     return ce;
 }
 
+bool reorder_fits(const slime_ensemble* e, const Colony& c) {
+    return c.n > 0 && reorder_scratch_bytes(c.n, c.W, c.H, e->reorder_cell_log2) > 0;
+}
+
 // Morton-reorder every colony's slots (results are unchanged: each slot keeps
 // its colony-local id).  With the lanes engine's lanes in place the colonies'
 // sorts run on four of them at once (largest first, each onto the lane with
 // the fewest agents so far), each of those lanes with its own sort scratch;
 // otherwise one after another on the ensemble's stream.  With `fitting` only
-// the colonies that launch_reorder takes.
+// the colonies that launch_reorder takes (reorder_fits).
 int reorder_all(slime_ensemble* e, bool fitting = false) {
     auto sorts = [&](const Colony& c) {
-        return c.n > 0 && (!fitting || reorder_fits(c.W, c.H, e->reorder_cell_log2));
+        return c.n > 0 && (!fitting || reorder_fits(e, c));
     };
     const size_t nr = e->lanes.size() < 4 ? e->lanes.size() : 4;
     cudaError_t ce = cudaSuccess;
@@ -609,7 +614,7 @@ int reorder_all(slime_ensemble* e, bool fitting = false) {
 uint64_t sortable_agents(const slime_ensemble* e) {
     uint64_t n = 0;
     for (const Colony& c : e->colonies)
-        if (reorder_fits(c.W, c.H, e->reorder_cell_log2)) n += c.n;
+        if (reorder_fits(e, c)) n += c.n;
     return n;
 }
 
@@ -620,6 +625,26 @@ uint32_t ens_sorted_steps(const slime_ensemble* e) {
     for (const Colony& c : e->colonies)
         if (c.n) steps = std::min(steps, sorted_steps_of(c.dev));
     return steps;
+}
+
+// Whether the scratch of a sort that no schedule asks for is there, or can come
+// from memory that is amply there (a quarter of what is free).  A lane's scratch
+// is its largest colony's, so the largest colonies' are what four lanes take.
+bool scratch_ready(const slime_ensemble* e) {
+    std::vector<size_t> need;
+    for (const Colony& c : e->colonies)
+        if (reorder_fits(e, c)) need.push_back(reorder_scratch_bytes(c.n, c.W, c.H, e->reorder_cell_log2));
+    std::sort(need.begin(), need.end(), std::greater<size_t>());
+    const size_t nr = e->engine == SLIME_ENSEMBLE_LANES && e->lanes.size() > 1 ? std::min<size_t>(e->lanes.size(), 4) : 1;
+    size_t more = 0;
+    for (size_t l = 0; l < nr && l < need.size(); l++) {
+        const ReorderScratch& scratch = l == 0 ? e->reorder : e->lane_reorder[l - 1];
+        if (scratch.bytes < need[l]) more += need[l];
+    }
+    size_t free_b = 0, total_b = 0;
+    if (more == 0) return true;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) cudaGetLastError();
+    return more <= free_b / 4;
 }
 
 // No scratch memory for a sort: the steps go on in the slots' order as it is,
@@ -638,7 +663,7 @@ int auto_sort(slime_ensemble* e, uint32_t n) {
     const bool due = e->sorted ? e->steps_done - e->sorted_since >= ens_sorted_steps(e)
                                : (uint64_t)n + e->unsorted_steps >= sorted_min_steps(sortable_agents(e));
     if (!due) return SLIME_OK;
-    const int rc = reorder_all(e, true);
+    const int rc = scratch_ready(e) ? reorder_all(e, true) : SLIME_ERR_OUT_OF_MEMORY;
     if (rc == SLIME_ERR_OUT_OF_MEMORY) {
         give_up_auto_sort(e);
         return SLIME_OK;
@@ -1210,7 +1235,7 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
                         e->stream);
     }
     if (e->reorder_every || (e->auto_sort && sorted_min_steps(sortable_agents(e)) < 1000)) { // as the steps will have them
-        int rrc = reorder_all(e, !e->reorder_every);
+        int rrc = e->reorder_every ? reorder_all(e) : (scratch_ready(e) ? reorder_all(e, true) : SLIME_ERR_OUT_OF_MEMORY);
         if (rrc == SLIME_OK && !e->reorder_every) {
             e->sorted = true;
             e->sorted_since = e->steps_done;

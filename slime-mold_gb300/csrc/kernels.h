@@ -149,8 +149,9 @@ struct ReorderScratch {
     size_t bytes = 0;
 };
 cudaError_t launch_iota(uint32_t* ids, uint64_t n, cudaStream_t s);
-// Whether a W x H trail has a Morton key of 32 bits (else launch_reorder refuses).
-bool reorder_fits(uint32_t W, uint32_t H, int cell_log2);
+// Bytes of scratch for n agents on a W x H trail (cell_log2 0 to 15), or 0 where a
+// side has more than 16 bits of key (launch_reorder refuses).
+size_t reorder_scratch_bytes(uint64_t n, uint32_t W, uint32_t H, int cell_log2);
 // The agents of `a` into `to` in Morton order (`to` may be `a` itself, with an id
 // array; without ids a's slots are the ids); agents with id >= `visited` go to
 // the last slots.  Six kernels.

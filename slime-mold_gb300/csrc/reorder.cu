@@ -13,8 +13,11 @@
 // five memory sectors an agent when the agents come unsorted, 160 bytes against
 // 64), and a pass that unpacks the records into the fields' arrays: the
 // agents' own, or another set, which is then sorted while the first stays as
-// it is.  The order inside one key is whatever the scatter atomics produce.  Agents whose id is
-// at or above `visited` (those the reference's dispatch never updates) get
+// it is.  A key has as many bits as the two sides need: where one side is longer
+// its upper bits stand above the interleaved ones (the order of the codes of a
+// square, whose unused bits are left out), so there are no more keys than four
+// times the squares of cells, however long and thin the trail.  The order inside
+// one key is whatever the scatter atomics produce.  Agents whose id is at or above `visited` (those the reference's dispatch never updates) get
 // one key past every Morton code, so they end up in the last slots and the
 // updated agents fill the first ones.
 #include "kernels.h"
@@ -41,12 +44,15 @@ __device__ __forceinline__ uint32_t spread_bits(uint32_t v) {
 // one key elect a leader that adds the group's size with a single atomic.
 __global__ void key_hist_kernel(const float* __restrict__ x, const float* __restrict__ y,
                                 const uint32_t* __restrict__ ids, uint64_t visited, uint32_t frozen_key, uint64_t n,
-                                int W, int H, int cl, uint32_t* __restrict__ keys, uint32_t* __restrict__ hist) {
+                                int W, int H, int cl, int low, uint32_t* __restrict__ keys,
+                                uint32_t* __restrict__ hist) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int cx = min(max(slm_f2i(x[i]), 0), W - 1) >> cl;
     int cy = min(max(slm_f2i(y[i]), 0), H - 1) >> cl;
-    uint32_t k = spread_bits((uint32_t)cx) | (spread_bits((uint32_t)cy) << 1);
+    const uint32_t mask = (1u << low) - 1u; // `low` bits of either side are interleaved
+    uint32_t k = spread_bits((uint32_t)cx & mask) | (spread_bits((uint32_t)cy & mask) << 1);
+    if (low < 16) k |= (((uint32_t)cx | (uint32_t)cy) >> low) << (2 * low);
     if (visited < n && (ids ? ids[i] : (uint32_t)i) >= visited) k = frozen_key;
     keys[i] = k;
     const unsigned group = __match_any_sync(__activemask(), k);
@@ -180,20 +186,33 @@ cudaError_t launch_iota(uint32_t* ids, uint64_t n, cudaStream_t s) {
 
 namespace {
 
-// Bits of the Morton key per side.
-int key_bits(uint32_t W, uint32_t H, int cell_log2) {
-    const uint32_t dx = (W + (1u << cell_log2) - 1) >> cell_log2;
-    const uint32_t dy = (H + (1u << cell_log2) - 1) >> cell_log2;
-    const uint32_t d = dx > dy ? dx : dy;
+// Bits of the sort key along a side.
+int key_bits(uint32_t side, int cell_log2) {
+    const uint32_t d = (side + (1u << cell_log2) - 1) >> cell_log2;
     int L = 0;
     while ((1u << L) < d) L++;
     return L;
 }
 
+struct ReorderSizes {
+    uint64_t keys, blocks; // histogram entries, and blocks that scan them
+    size_t bytes;          // of scratch
+};
+ReorderSizes reorder_sizes(uint64_t n, uint32_t W, uint32_t H, int cell_log2, bool partition) {
+    ReorderSizes r;
+    r.keys = (1ull << (key_bits(W, cell_log2) + key_bits(H, cell_log2))) + (partition ? 1 : 0);
+    r.blocks = (r.keys + kScanTile - 1) / kScanTile;
+    r.bytes = align256(4 * n) /*keys*/ + align256(4 * r.keys) /*histogram*/ + align256(4 * r.blocks) /*block sums*/ +
+              align256(16 * n) /*records*/ + align256(4 * n) /*ids*/;
+    return r;
+}
+
 } // namespace
 
-bool reorder_fits(uint32_t W, uint32_t H, int cell_log2) {
-    return key_bits(W, H, cell_log2) <= 16;
+size_t reorder_scratch_bytes(uint64_t n, uint32_t W, uint32_t H, int cell_log2) {
+    const int lx = key_bits(W, cell_log2), ly = key_bits(H, cell_log2);
+    if (lx > 16 || ly > 16) return 0;
+    return reorder_sizes(n, W, H, cell_log2, false).bytes;
 }
 
 cudaError_t launch_reorder(const AgentsSoA& a, const AgentsSoA& to, uint32_t W, uint32_t H, int cell_log2,
@@ -202,16 +221,15 @@ cudaError_t launch_reorder(const AgentsSoA& a, const AgentsSoA& to, uint32_t W, 
     if (!to.ids) return cudaErrorInvalidValue;
     if (cell_log2 < 0) cell_log2 = 0;
     if (cell_log2 > 15) cell_log2 = 15;
-    const int L = key_bits(W, H, cell_log2);
-    if (L > 16) return cudaErrorInvalidValue;
+    const int lx = key_bits(W, cell_log2), ly = key_bits(H, cell_log2);
+    if (lx > 16 || ly > 16) return cudaErrorInvalidValue;
     const bool partition = visited < a.n;
-    if (partition && L > 15) return cudaErrorInvalidValue; // no key left past the Morton codes
-    const uint32_t frozen_key = (uint32_t)(1ull << (2 * L));
-    uint64_t nb = (1ull << (2 * L)) + (partition ? 1 : 0);
-    uint64_t nblk = (nb + kScanTile - 1) / kScanTile;
+    if (partition && (lx > 15 || ly > 15)) return cudaErrorInvalidValue; // no key left past the Morton codes
+    const uint32_t frozen_key = (uint32_t)(1ull << (lx + ly));
     const uint64_t n = a.n;
-    size_t need = align256(4 * n) /*keys*/ + align256(4 * nb) /*hist*/ + align256(4 * nblk) /*block sums*/ +
-                  align256(16 * n) /*records*/ + align256(4 * n) /*ids*/;
+    const ReorderSizes size = reorder_sizes(n, W, H, cell_log2, partition);
+    const uint64_t nb = size.keys, nblk = size.blocks;
+    const size_t need = size.bytes;
     if (scratch.bytes < need) {
         if (scratch.buf) dev_free(scratch.buf);
         scratch.buf = nullptr;
@@ -230,8 +248,8 @@ cudaError_t launch_reorder(const AgentsSoA& a, const AgentsSoA& to, uint32_t W, 
     cudaError_t e = cudaMemsetAsync(hist, 0, 4 * nb, s);
     if (e != cudaSuccess) return e;
     unsigned blocks = (unsigned)((n + 255) / 256);
-    key_hist_kernel<<<blocks, 256, 0, s>>>(a.x, a.y, a.ids, visited, frozen_key, n, (int)W, (int)H, cell_log2, keys,
-                                          hist);
+    key_hist_kernel<<<blocks, 256, 0, s>>>(a.x, a.y, a.ids, visited, frozen_key, n, (int)W, (int)H, cell_log2, lx < ly ? lx : ly,
+                                          keys, hist);
     scan_reduce_kernel<<<(unsigned)nblk, kScanThreads, 0, s>>>(hist, nb, bsum);
     scan_block_sums_kernel<<<1, kScanThreads, 0, s>>>(bsum, (uint32_t)nblk);
     scan_apply_kernel<<<(unsigned)nblk, kScanThreads, 0, s>>>(hist, nb, bsum);

@@ -292,7 +292,8 @@ struct slime_ensemble {
     ReorderScratch lane_reorder[3]; // sort scratch of the lanes engine's concurrent reorders (with `reorder`)
     float* trail[2] = {nullptr, nullptr};
     uint32_t* counts[2] = {nullptr, nullptr};
-    uint8_t* marks[2] = {nullptr, nullptr}; // per-cell deposit marks (lanes engine; allocated on first use)
+    uint8_t* marks[2] = {nullptr, nullptr}; // per-cell deposit marks (lanes engine; both allocated on first use)
+    bool marks_refused = false;             // there was no memory for them
     int cur = 0;
     DevColony* d_cols = nullptr;
     uint2* d_agent_items = nullptr;
@@ -691,8 +692,25 @@ int check_barrier(slime_ensemble* e) {
 // the cell to 1, so whether a cell received any carries the fold), and at most
 // one agent per cell (use_marks in capi.cu).
 bool colony_marks(const slime_ensemble* e, const Colony& c) {
-    return e->engine == SLIME_ENSEMBLE_LANES && c.n > 0 && c.n <= (uint64_t)c.W * c.H && c.trail_clean && c.dev.dep >= 1.0f &&
-           keeps_trail_clean(c.dev) && trail_tile_streams(c.dev, e->lane_trail_tile);
+    return e->engine == SLIME_ENSEMBLE_LANES && !e->marks_refused && c.n > 0 && c.n <= (uint64_t)c.W * c.H &&
+           c.trail_clean && c.dev.dep >= 1.0f && keeps_trail_clean(c.dev) && trail_tile_streams(c.dev, e->lane_trail_tile);
+}
+
+// Both mark arrays, or none: without memory for them the colonies count.
+void alloc_marks(slime_ensemble* e) {
+    cudaError_t ce = cudaSuccess;
+    for (int i = 0; i < 2 && ce == cudaSuccess; i++) {
+        ce = dev_alloc((void**)&e->marks[i], e->total_cells);
+        if (ce == cudaSuccess) ce = cudaMemsetAsync(e->marks[i], 0, e->total_cells, e->stream);
+    }
+    for (Colony& c : e->colonies) c.marks_dirty[0] = c.marks_dirty[1] = false;
+    if (ce == cudaSuccess) return;
+    cudaGetLastError();
+    for (int i = 0; i < 2; i++) {
+        dev_free(e->marks[i]);
+        e->marks[i] = nullptr;
+    }
+    e->marks_refused = true;
 }
 
 // Before a chunk: each colony's record kind (a change drops the captured
@@ -701,6 +719,8 @@ bool colony_marks(const slime_ensemble* e, const Colony& c) {
 // other engine left deposits in it.
 int prepare_ens_deposits(slime_ensemble* e) {
     bool changed = false;
+    for (const Colony& c : e->colonies)
+        if (!e->marks[0] && colony_marks(e, c)) alloc_marks(e);
     for (Colony& c : e->colonies) {
         const bool mk = colony_marks(e, c);
         changed = changed || mk != c.marks;
@@ -711,13 +731,6 @@ int prepare_ens_deposits(slime_ensemble* e) {
     for (Colony& c : e->colonies) {
         const size_t cells = (size_t)c.W * c.H;
         if (c.marks) {
-            if (!e->marks[0]) {
-                for (int i = 0; i < 2; i++) {
-                    ECK(dev_alloc((void**)&e->marks[i], e->total_cells), "allocating deposit marks");
-                    ECK(cudaMemsetAsync(e->marks[i], 0, e->total_cells, e->stream), "clearing deposit marks");
-                }
-                for (Colony& o : e->colonies) o.marks_dirty[0] = o.marks_dirty[1] = false;
-            }
             if (c.marks_dirty[cur]) {
                 ECK(cudaMemsetAsync(e->marks[cur] + c.trail_off, 0, cells, e->stream), "clearing deposit marks");
                 c.marks_dirty[cur] = false;
@@ -1187,6 +1200,7 @@ int slime_ensemble_set_engine(slime_ensemble* e, uint32_t engine, uint32_t agent
     cudaSetDevice(e->device);
     ECK(cudaStreamSynchronize(e->stream), "synchronising");
     e->engine = (int)engine;
+    e->marks_refused = false; // asked for again
     e->lane_agent_shape = (int)agent_shape;
     e->lane_trail_tile = (int)trail_tile;
     ens_invalidate(e);

@@ -107,3 +107,29 @@ def test_colonies_too_wide_to_sort_step(gpu, engine, tuned):
     ens.set_reorder(5, 2)
     with pytest.raises(sg.SlimeError):
         ens.step(5)
+
+
+# Agents, ids and the upload's buffer are 36 bytes an agent, the trails and
+# counts 16 a cell, and two arrays of marks one a cell each: not even one of
+# them fits, or one.
+@pytest.mark.parametrize("spare", [150_000, 420_000])
+def test_steps_without_memory_for_marks(gpu, tmp_path, spare):
+    import slime_gb300 as sg
+    side, n = 512, 20_000
+    code = f"""
+S, n = {side}, {n}
+ens = sg.Ensemble([S], [S], [n], [config0_params(S, S)])
+ens.upload_agents(0, agents_uniform(n, S, S, 1.0, 2.0, seed=1))
+ens.step(3)
+ens.step(20)
+np.savez({str(tmp_path / "out.npz")!r}, a=ens.download_agents(0), t=ens.download_trail(0),
+         marks=ens.info().marks_colonies, engine=ens.info().engine)
+"""
+    capped(code, 36 * n + 16 * side * side + spare)
+    got = np.load(tmp_path / "out.npz")
+    assert got["engine"] == sg.ENSEMBLE_LANES and got["marks"] == 0
+    with sg.Simulation(side, side, n, config0_params(side, side)) as sim:
+        sim.upload_agents(agents_uniform(n, side, side, 1.0, 2.0, seed=1))
+        sim.step(23)
+        assert_bitexact(got["a"], sim.download_agents(), "agents")
+        assert_bitexact(got["t"], sim.download_trail(), "trail")

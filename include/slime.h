@@ -376,7 +376,8 @@ int slime_ensemble_set_engine(slime_ensemble* ens, uint32_t engine, uint32_t lan
 /* Choose the cooperative step's launch shape by hand (what slime_ensemble_autotune picks
  * by timing): trail rows per strip item (8, 16 or 32), resident blocks per SM
  * (0 = as many as fit, else 1..4) and agents per thread of the agent phase
- * (4: each stepped alone; 2: stepped as one pair).  Results do not change. */
+ * (4: each stepped alone; 2: stepped as one pair).  An ensemble whose engine was
+ * neither chosen nor tuned steps cooperatively then.  Results do not change. */
 int slime_ensemble_set_shape(slime_ensemble* ens, uint32_t strip_rows, uint32_t blocks_per_sm,
                              uint32_t agents_per_thread);
 /* Total kernels enqueued so far. */

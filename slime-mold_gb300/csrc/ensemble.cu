@@ -312,6 +312,7 @@ struct slime_ensemble {
     bool use_graphs = true;
     bool last_chunk_graph = false; // the last chunk of steps replayed a graph
     int engine = SLIME_ENSEMBLE_COOPERATIVE;
+    bool engine_chosen = false; // by hand, by its shape or by the autotuner
     int lane_agent_shape = 13; // agent-kernel shape of the lanes engine (persistent, texture gather)
     int lane_trail_tile = 8;   // trail tile of the lanes engine (streaming, 16-row strips)
     int max_lanes = 0;         // lanes of the lanes engine (0: one per colony, at most 64)
@@ -1200,6 +1201,7 @@ int slime_ensemble_set_engine(slime_ensemble* e, uint32_t engine, uint32_t agent
     cudaSetDevice(e->device);
     ECK(cudaStreamSynchronize(e->stream), "synchronising");
     e->engine = (int)engine;
+    e->engine_chosen = true;
     e->marks_refused = false; // asked for again
     e->lane_agent_shape = (int)agent_shape;
     e->lane_trail_tile = (int)trail_tile;
@@ -1221,6 +1223,8 @@ int slime_ensemble_set_shape(slime_ensemble* e, uint32_t strip_rows, uint32_t bl
     }
     cudaSetDevice(e->device);
     ECK(cudaStreamSynchronize(e->stream), "synchronising");
+    if (!e->engine_chosen) e->engine = SLIME_ENSEMBLE_COOPERATIVE; // whose shape this is
+    e->engine_chosen = true;
     e->rows = (int)strip_rows;
     e->blocks_per_sm = (int)blocks_per_sm;
     e->apt = (int)agents_per_thread;
@@ -1379,6 +1383,7 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
     e->blocks_per_sm = best_bps;
     e->apt = best_apt;
     e->engine = best_engine;
+    e->engine_chosen = true;
     e->lane_agent_shape = best_shape;
     e->lane_trail_tile = best_tile;
     ens_invalidate(e);

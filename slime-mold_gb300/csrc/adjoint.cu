@@ -30,36 +30,29 @@ namespace {
 
 // One backward step.  A block takes a tile of 128 x 16 cells, a thread four
 // adjacent columns of every fourth row, and stages the window of u (T_s folded
-// and decayed) and of g with 16-byte loads.  What bounded it before were the
-// block's sums (three binary64 butterflies over all its threads, on a GPU with
-// two binary64 operations per SM and cycle), a second read of T and k for the
-// thread's own cells, and one cell per thread per pass through shared memory:
-//   * a thread sums each of its columns' four cells in binary32, and keeps its
-//     three sums over all steps as unevaluated binary32 pairs in memory
-//     (T. Dekker, "A floating-point technique for extending the available
-//     precision", Numer. Math. 18, 1971: what an addition rounds off goes into
-//     the second number); they are added up in binary64 once per backward, in
-//     one order, so the gradients do not depend on which block finishes first;
+// and decayed) and of g with 16-byte loads.  A block that reads T and k a second
+// time for its own cells, blurs one cell per thread and adds its three sums up in
+// every step (binary64 butterflies over all its threads, on a GPU with two
+// binary64 operations per SM and cycle) is bound by those, so
+//   * a thread sums each of its columns' four cells in binary32 and adds those
+//     to its three sums over all steps, in binary64 and in memory; all threads'
+//     are added up once per backward, in one order, so the gradients do not
+//     depend on which block finishes first;
 //   * a thread's own cells of T and k are read once (with a shared-memory
 //     carve-out this large nothing stays in L1 for a second read), folded once
 //     and kept in registers, as is its g;
 //   * u is staged before the wait for the step it follows, which writes only g.
 // The blur of g is separable; B(u) - u, small against u, is summed term by term
-// from neighbour-minus-centre differences.  Sum by sum the arithmetic of the
-// kernel before: 1024^2, radius 1, 22.6 us a step then, 8.7 now (16.8 MB
-// of T, k and g: 2.5 us at the measured copy bandwidth).
+// from neighbour-minus-centre differences.  Cell for cell the arithmetic of a
+// block that sums over all its threads in every step: 1024^2, radius 1, 22.6 us a
+// step so and 11.0 here (16.8 MB of T, k and g: 2.5 us at the measured copy
+// bandwidth).  2.3 of the 11.0 are the twelve binary64 additions and conversions
+// a thread; sums kept as pairs of binary32 numbers did without, in 48 bits and
+// binary32's range.  Conversions by integer operations measure the same.
 constexpr int kTW = 128, kTH = 16;
 constexpr int kSlots = 4;              // a thread's rows are its slot and every fourth after it
 constexpr int kRows = kTH / kSlots;
 constexpr int kThreads = kTW / 4 * kSlots;
-
-// s.x + s.y += x: what the sum s.x + x rounds off (Knuth's two-sum) joins s.y.
-__device__ __forceinline__ void pair_add(float2& s, float x) {
-    const float t = slm_add(s.x, x);
-    const float b = slm_sub(t, s.x);
-    s.y = slm_add(s.y, slm_add(slm_sub(s.x, slm_sub(t, b)), slm_sub(x, b)));
-    s.x = t;
-}
 
 // The first n of four cells from i.
 __device__ __forceinline__ float4 row4(const float* __restrict__ a, size_t i, int n) {
@@ -100,7 +93,7 @@ __device__ __forceinline__ float4 folded(const DevParams& p, const float4& t, co
 template <int R, bool kGauss>
 __global__ void __launch_bounds__(kThreads) adjoint_kernel(const __grid_constant__ DevParams p,
                                                            const float* __restrict__ T, const uint32_t* __restrict__ K,
-                                                           const float* gin, float* gout, float2* acc,
+                                                           const float* gin, float* gout, double* acc,
                                                            uint32_t rate_active, int tiles_x, int vec) {
     typedef TileGeom<kTW, kTH, R> G; // window layout
     constexpr int NH = (2 * R + kSlots - 1) / kSlots; // halo rows per slot
@@ -182,8 +175,8 @@ __global__ void __launch_bounds__(kThreads) adjoint_kernel(const __grid_constant
     // g and the sums are the output of the step this one follows
     pdl_wait();
     pdl_trigger();
-    float2* own_acc = acc + (size_t)blockIdx.x * (3 * kThreads) + threadIdx.x;
-    float2 s[3] = {own_acc[0], own_acc[kThreads], own_acc[2 * kThreads]};
+    double* own_acc = acc + (size_t)blockIdx.x * (3 * kThreads) + threadIdx.x;
+    double s[3] = {own_acc[0], own_acc[kThreads], own_acc[2 * kThreads]};
     if (vec) {
         float4 gh[NH > 0 ? NH : 1];
 #pragma unroll
@@ -333,9 +326,9 @@ __global__ void __launch_bounds__(kThreads) adjoint_kernel(const __grid_constant
     }
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        pair_add(s[0], sd[j]);
-        pair_add(s[1], sr[j]);
-        pair_add(s[2], sp[j]);
+        s[0] += (double)sd[j];
+        s[1] += (double)sr[j];
+        s[2] += (double)sp[j];
     }
     own_acc[0] = s[0];
     own_acc[kThreads] = s[1];
@@ -355,14 +348,11 @@ __device__ __forceinline__ double block_sum(double v) {
     }
     return s[0];
 }
-__global__ void __launch_bounds__(kThreads) sum_threads_kernel(const float2* __restrict__ acc, uint32_t blocks,
+__global__ void __launch_bounds__(kThreads) sum_threads_kernel(const double* __restrict__ acc, uint32_t blocks,
                                                           double* __restrict__ part) {
     double v = 0.0;
-    for (uint32_t b = blockIdx.x; b < blocks; b += kSumBlocks) {
-        const float2 a = acc[((size_t)b * 3 + blockIdx.y) * kThreads + threadIdx.x];
-        // an infinite or NaN sum says nothing in its second number
-        v += (double)a.x + (fabsf(a.x) <= 3.0e38f ? (double)a.y : 0.0);
-    }
+    for (uint32_t b = blockIdx.x; b < blocks; b += kSumBlocks)
+        v += acc[((size_t)b * 3 + blockIdx.y) * kThreads + threadIdx.x];
     v = block_sum(v);
     if (threadIdx.x == 0) part[blockIdx.y * kSumBlocks + blockIdx.x] = v;
 }
@@ -377,7 +367,7 @@ uint32_t adjoint_blocks(uint32_t W, uint32_t H) {
 
 template <int R, bool kGauss>
 cudaError_t launch_adj(const DevParams& p, const float* T, const uint32_t* K, const float* gin, float* gout,
-                       float2* acc, uint32_t rate_active, cudaStream_t s, bool pdl) {
+                       double* acc, uint32_t rate_active, cudaStream_t s, bool pdl) {
     typedef TileGeom<kTW, kTH, R> G;
     const size_t smem = sizeof(float) * (2 * G::window + (kGauss ? G::SH * kTW : 0));
     if (smem > 48 * 1024) {
@@ -393,7 +383,7 @@ cudaError_t launch_adj(const DevParams& p, const float* T, const uint32_t* K, co
 } // namespace
 
 cudaError_t launch_adjoint_step(const DevParams& p, const float* T, const uint32_t* K, const float* gin,
-                                float* gout, float2* acc, uint32_t rate_active, cudaStream_t s, bool pdl) {
+                                float* gout, double* acc, uint32_t rate_active, cudaStream_t s, bool pdl) {
     if (p.blur_mode != SLIME_BLUR_GAUSS) return launch_adj<1, false>(p, T, K, gin, gout, acc, rate_active, s, pdl);
     switch (p.R) {
     case 0: return launch_adj<0, true>(p, T, K, gin, gout, acc, rate_active, s, pdl);
@@ -465,7 +455,7 @@ size_t segment_stride(const slime_ctx* ctx) { return ((size_t)ctx->W * ctx->H + 
 
 size_t acc_bytes(const slime_ctx* ctx) {
     return (4 + 3 * kSumBlocks) * sizeof(double) +
-           (size_t)adjoint_blocks(ctx->W, ctx->H) * 3 * kThreads * sizeof(float2);
+           (size_t)adjoint_blocks(ctx->W, ctx->H) * 3 * kThreads * sizeof(double);
 }
 
 // The buffers of the backward, as the recording's sizes have them: all of them
@@ -701,7 +691,7 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
        "uploading dL/dT");
     CK(cudaMemsetAsync(a.acc, 0, acc_bytes(ctx), ctx->stream), "clearing gradients");
     double* parts = (double*)a.acc;                      // 3, then 3 x kSumBlocks, then every thread's
-    float2* thread_acc = (float2*)(parts + 4 + 3 * kSumBlocks);
+    double* thread_acc = parts + 4 + 3 * kSumBlocks;
     int cg = 0;
     AgentsSoA tmp;
     tmp.x = a.agents_tmp;

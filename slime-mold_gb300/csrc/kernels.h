@@ -136,10 +136,10 @@ int trail_tma_misaligned_blocks();
 // One backward step of the frozen-trajectory chain: from g_in = dL/dT_{s+1}
 // and the step's input trail T_s and counts k_s, writes g_out = dL/dT_s and
 // adds the step's parameter-gradient contributions to every thread's own sums
-// in acc (decay_factor, diffusion_rate, deposition).  With `pdl` it follows
+// in acc, in binary64 (decay_factor, diffusion_rate, deposition).  With `pdl` it follows
 // another backward step, and its T and k were complete before that one began.
 cudaError_t launch_adjoint_step(const DevParams& p, const float* trail_s, const uint32_t* counts_s,
-                                const float* g_in, float* g_out, float2* acc, uint32_t rate_active,
+                                const float* g_in, float* g_out, double* acc, uint32_t rate_active,
                                 cudaStream_t s, bool pdl);
 
 // ---- reorder.cu

@@ -575,8 +575,8 @@ SLM_FN uint32_t slm_dispatch_visits(uint64_t n, uint64_t index) {
 /* slm_sincos of two arguments with |x0|, |x1| < 4096 at once, bit for bit.
  * Each lane's reduction starts with a binary32 product and sum (a packed
  * product followed by a packed sum may be contracted into one fused
- * operation, which would round once instead of twice, so the sums stay
- * scalar); every later step is a fused multiply-add, or a product that feeds
+ * operation, which would round once instead of twice; into scalar sums it is
+ * not, so the sums stay scalar); every later step is a fused multiply-add, or a product that feeds
  * one as a multiplicand, evaluated for both lanes by one packed instruction
  * (fma.rn.f32x2, mul.rn.f32x2: each lane rounded as its scalar form). */
 static __device__ __forceinline__ void slm_sincos2_cw(float x0, float x1, float* s0, float* c0, float* s1,

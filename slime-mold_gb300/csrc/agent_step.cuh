@@ -218,9 +218,11 @@ __device__ __forceinline__ int agent_step(const DevParams& p, float& x, float& y
 // directions, jitter hashes, moves) paired into packed fused multiply-adds,
 // as are each agent's two side directions, and packed products, sums and
 // differences where a pair's operands lie side by side (the sensor positions,
-// the fractions and weights of a footprint, the hash's products): at 4096^2 the
-// agent pass takes 203.3 us with them and 206.9 without.  Bit for bit agent_step
-// twice.
+// the fractions and weights of a footprint, the hash's products).  Agent pass at
+// 4096^2 with those / with them scalar, us: shape 13, the default, 211.4 / 212.3,
+// rotated sensors 199.2 / 200.2; shape 14 211.5 / 214.5 and 206.5 / 207; shape 15,
+// held to four blocks an SM, 231.7 / 225.8 and 221.6 / 215.4.  Bit for bit
+// agent_step twice.
 // The two agents' sensor directions (centre, left, right), (cos, sin) each.
 struct SensorDirs2 {
     float cca, sca, ccb, scb, cla, sla, cra, sra, clb, slb, crb, srb;

@@ -285,7 +285,10 @@ int slime_get_stream(slime_ctx* ctx, void** stream);
  * runtime performs it synchronously. */
 int slime_download_trail_async(slime_ctx* ctx, float* trail, uint64_t n_cells);
 int slime_wait_download(slime_ctx* ctx);
-/* Deposit counts of the most recent step (cells receiving k agents hold k). */
+/* Deposit counts of the most recent step (cells receiving k agents hold k).
+ * Without options.exact_counts they are refused (SLIME_ERR_STATE) after a step
+ * whose deposits all saturate the fold on a streaming trail tile that was
+ * chosen or tuned. */
 int slime_download_deposit_counts(slime_ctx* ctx, uint32_t* counts, uint64_t n_cells);
 /* Reorder agents in Morton order of their cell now (results are unchanged:
  * every agent keeps its id, which seeds its jitter hash). */

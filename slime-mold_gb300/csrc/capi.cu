@@ -1470,8 +1470,8 @@ int slime_download_deposit_counts(slime_ctx* ctx, uint32_t* counts, uint64_t n_c
     }
     if (ctx->last_no_counts)
         return set_error(ctx->err, SLIME_ERR_STATE,
-                         "the last step recorded which cells received deposits, not how many (every deposit "
-                         "saturated the fold); set options.exact_counts = 1 to keep counts");
+                         "a streaming trail tile that was chosen or tuned keeps no deposit counts while every "
+                         "deposit saturates the fold; set options.exact_counts = 1 to keep them");
     const int rc = make_counts(ctx);
     if (rc != SLIME_OK) return rc;
     CK(cudaMemcpyAsync(counts, ctx->counts[1 - ctx->cur], n_cells * sizeof(uint32_t), cudaMemcpyDeviceToHost,

@@ -609,7 +609,8 @@ int record_steps(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) {
         return cuda_error(ctx->err, e, "allocating checkpoints");
     }
     for (uint32_t j = 0; j < a.n_ckpt; j++) {
-        int rc = resort_run(ctx);
+        uint32_t m = (n_steps - j * K) < K ? (n_steps - j * K) : K;
+        int rc = resort_run(ctx, m);
         if (rc != SLIME_OK) return rc;
         CK(cudaMemcpyAsync(a.ckpt_agents + (size_t)j * 4 * n_pad, ctx->agents.x, 4 * n_pad * sizeof(float),
                            cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing agents");
@@ -618,7 +619,6 @@ int record_steps(slime_ctx* ctx, uint32_t n_steps, uint32_t ckpt_every) {
                                cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing ids");
         CK(cudaMemcpyAsync(a.ckpt_trail + (size_t)j * cells, ctx->trail[ctx->cur], cells * sizeof(float),
                            cudaMemcpyDeviceToDevice, ctx->stream), "checkpointing trail");
-        uint32_t m = (n_steps - j * K) < K ? (n_steps - j * K) : K;
         if (j + 1 == a.n_ckpt && segment_ready(ctx)) {
             if ((rc = record_last_segment(ctx, m)) != SLIME_OK) return rc;
             a.seg_holds = (int)j;

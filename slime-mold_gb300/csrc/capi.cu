@@ -725,10 +725,9 @@ bool sorted_run_ready(slime_ctx* ctx, uint32_t n_steps) {
     return true;
 }
 
-// Before n_steps steps: onto the copy where that pays, the copy sorted again
-// where its order has aged.
+// Before n_steps steps: onto the copy where that pays.
 int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps) {
-    if (ctx->in_sorted_run) return resort_run(ctx);
+    if (ctx->in_sorted_run) return SLIME_OK;
     if (!sorted_run_ready(ctx, n_steps)) return SLIME_OK;
     AgentsSoA to = ctx->agents;
     to.x = (float*)ctx->sorted_block;
@@ -752,9 +751,17 @@ int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps) {
     return SLIME_OK;
 }
 
-// Between steps on the copy: sort it again when its order has aged.
-int resort_run(slime_ctx* ctx) {
-    if (!ctx->in_sorted_run || ctx->steps_done - ctx->sorted_since < sorted_steps(ctx)) return SLIME_OK;
+// Whether agents sorted `age` steps ago are sorted before the next `take` steps:
+// when those would end further past `interval` than it is away.  Chunks of steps
+// are not cut for a sort, whose place would differ from call to call: a graph of
+// almost any length would be captured and kept.
+bool resort_due(uint64_t age, uint32_t take, uint32_t interval) {
+    return age > 0 && 2 * age + take >= 2 * (uint64_t)interval;
+}
+
+// Before `take` steps on the copy: sort it again when its order has aged.
+int resort_run(slime_ctx* ctx, uint32_t take) {
+    if (!ctx->in_sorted_run || !resort_due(ctx->steps_done - ctx->sorted_since, take, sorted_steps(ctx))) return SLIME_OK;
     CK(launch_reorder(ctx->agents, ctx->agents, ctx->W, ctx->H, 2, ctx->reorder, ctx->stream), "sorting agents");
     ctx->launches += kReorderKernels;
     ctx->sorted_since = ctx->steps_done;
@@ -891,16 +898,22 @@ int ensure_dispatch_order(slime_ctx* ctx) {
     return do_reorder(ctx);
 }
 
+// How many of the next n steps are made at once: a graph's, and on the sorted
+// copy no more than it stays in order.
+uint32_t chunk_of(const slime_ctx* ctx, uint32_t n) {
+    const uint32_t chunk = ctx->opt.graph_chunk ? ctx->opt.graph_chunk : 50;
+    if (ctx->opt.use_graphs && chunk < n) n = chunk;
+    if (ctx->in_sorted_run && sorted_steps(ctx) < n) n = sorted_steps(ctx);
+    return n;
+}
+
 // Capture the graphs that the next n steps replay (same chunking as
-// run_steps: graph_chunk steps, cut at reorder boundaries), without stepping.
+// run_steps: chunk_of, cut at reorder boundaries), without stepping.
 int prepare_steps(slime_ctx* ctx, uint32_t n) {
     if (!ctx->opt.use_graphs || ctx->agents.n == 0) return SLIME_OK;
     int brc = begin_sorted_run(ctx, n); // the graphs step the copy, then
     if (brc != SLIME_OK) return brc;
-    const uint32_t aged = ctx->in_sorted_run ? sorted_steps(ctx) : ~0u;
-    uint32_t age = ctx->in_sorted_run ? (uint32_t)(ctx->steps_done - ctx->sorted_since) : 0u;
     const bool marks = use_marks(ctx);
-    const uint32_t chunk = ctx->opt.graph_chunk ? ctx->opt.graph_chunk : 50;
     const int saved = ctx->cur;
     uint64_t steps = ctx->steps_done;
     int rc = SLIME_OK;
@@ -910,14 +923,11 @@ int prepare_steps(slime_ctx* ctx, uint32_t n) {
             uint64_t to_next = ctx->opt.reorder_every - steps % ctx->opt.reorder_every;
             if (to_next < m) m = (uint32_t)to_next;
         }
-        if (age >= aged) age = 0;
-        if (aged - age < m) m = aged - age;
-        const uint32_t take = m < chunk ? m : chunk;
+        const uint32_t take = chunk_of(ctx, m);
         cudaGraphExec_t exec = nullptr;
         rc = step_graph(ctx, take, marks, &exec);
         if (take & 1) ctx->cur = 1 - ctx->cur;
         steps += take;
-        age += take;
         n -= take;
     }
     ctx->cur = saved;
@@ -927,31 +937,21 @@ int prepare_steps(slime_ctx* ctx, uint32_t n) {
 static int run_steps_on(slime_ctx* ctx, uint32_t n) {
     int rc;
     while (n > 0) {
-        if ((rc = resort_run(ctx)) != SLIME_OK) return rc;
         uint32_t m = n;
-        if (ctx->in_sorted_run) {
-            const uint64_t left = sorted_steps(ctx) - (ctx->steps_done - ctx->sorted_since);
-            if (left < m) m = (uint32_t)left;
-        }
         if (ctx->opt.reorder_every) {
             if (ctx->steps_done % ctx->opt.reorder_every == 0 && ctx->last_reorder_step != ctx->steps_done)
                 if ((rc = do_reorder(ctx)) != SLIME_OK) return rc;
             uint64_t to_next = ctx->opt.reorder_every - ctx->steps_done % ctx->opt.reorder_every;
             if (to_next < m) m = (uint32_t)to_next;
         }
+        const uint32_t take = chunk_of(ctx, m);
+        if ((rc = resort_run(ctx, take)) != SLIME_OK) return rc;
         const bool marks = use_marks(ctx);
         if ((rc = prepare_deposits(ctx, marks)) != SLIME_OK) return rc;
-        if (ctx->opt.use_graphs) {
-            uint32_t chunk = ctx->opt.graph_chunk ? ctx->opt.graph_chunk : 50;
-            uint32_t take = m < chunk ? m : chunk;
-            if ((rc = run_steps_graph(ctx, take, marks)) != SLIME_OK) return rc;
-            after_steps(ctx, marks, take);
-            n -= take;
-        } else {
-            if ((rc = run_steps_direct(ctx, m, marks)) != SLIME_OK) return rc;
-            after_steps(ctx, marks, m);
-            n -= m;
-        }
+        rc = ctx->opt.use_graphs ? run_steps_graph(ctx, take, marks) : run_steps_direct(ctx, take, marks);
+        if (rc != SLIME_OK) return rc;
+        after_steps(ctx, marks, take);
+        n -= take;
     }
     return SLIME_OK;
 }

@@ -154,7 +154,8 @@ int step_graph(slime_ctx* ctx, uint32_t m, bool marks, cudaGraphExec_t* out);
 int run_steps_direct(slime_ctx* ctx, uint32_t m, bool marks);
 int run_steps_graph(slime_ctx* ctx, uint32_t m, bool marks);
 int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps);
-int resort_run(slime_ctx* ctx);
+int resort_run(slime_ctx* ctx, uint32_t take);
+bool resort_due(uint64_t age, uint32_t take, uint32_t interval);
 int end_sorted_run(slime_ctx* ctx);
 void drop_sorted_run(slime_ctx* ctx);
 void release_sorted(slime_ctx* ctx);

@@ -657,14 +657,28 @@ void give_up_auto_sort(slime_ensemble* e) {
     e->err.clear();
 }
 
-// Before n steps: sort the colonies where that pays (the bounds of a single
-// context's copy, on the agents of all that can be sorted): 16 colonies of 256^2 to 1024^2 take 258
-// us a step sorted and 543 in no order.  Without scratch memory it is given up.
-int auto_sort(slime_ensemble* e, uint32_t n) {
-    if (e->reorder_every || !e->auto_sort) return SLIME_OK;
-    const bool due = e->sorted ? e->steps_done - e->sorted_since >= ens_sorted_steps(e)
-                               : (uint64_t)n + e->unsorted_steps >= sorted_min_steps(sortable_agents(e));
-    if (!due) return SLIME_OK;
+// Whether the next n steps are made on sorted colonies without a schedule: where
+// that pays (the bounds of a single context's copy, on the agents of all that can
+// be sorted; 16 colonies of 256^2 to 1024^2 take 258 us a step sorted and 543 in no
+// order).
+bool sorts_itself(const slime_ensemble* e, uint32_t n) {
+    return !e->reorder_every && e->auto_sort &&
+           (e->sorted || (uint64_t)n + e->unsorted_steps >= sorted_min_steps(sortable_agents(e)));
+}
+
+constexpr uint32_t kEnsChunk = 50;
+
+// How many of the next n steps are made at once (chunk_of in capi.cu).
+uint32_t ens_chunk_of(const slime_ensemble* e, uint32_t n, bool sorting) {
+    if (sorting) n = std::min(n, ens_sorted_steps(e));
+    return std::min(n, kEnsChunk);
+}
+
+// Before the next `take` of n steps: sort the colonies where that pays, again
+// when their order has aged.  Without scratch memory it is given up.
+int auto_sort(slime_ensemble* e, uint32_t n, uint32_t take) {
+    if (!sorts_itself(e, n)) return SLIME_OK;
+    if (e->sorted && !resort_due(e->steps_done - e->sorted_since, take, ens_sorted_steps(e))) return SLIME_OK;
     const int rc = scratch_ready(e) ? reorder_all(e, true) : SLIME_ERR_OUT_OF_MEMORY;
     if (rc == SLIME_ERR_OUT_OF_MEMORY) {
         give_up_auto_sort(e);
@@ -785,8 +799,6 @@ cudaGraphExec_t chunk_graph(slime_ensemble* e, uint32_t m) {
     return exec;
 }
 
-constexpr uint32_t kEnsChunk = 50;
-
 // Capture the graphs that the next n steps replay (run_ens_steps' chunks).
 int prepare_ens_steps(slime_ensemble* e, uint32_t n) {
     const bool lanes = e->engine == SLIME_ENSEMBLE_LANES;
@@ -801,18 +813,12 @@ int prepare_ens_steps(slime_ensemble* e, uint32_t n) {
     if (rc != SLIME_OK) return rc;
     const int saved = e->cur;
     uint64_t steps = e->steps_done;
-    const uint64_t agents = sortable_agents(e);
-    const uint32_t aged = ens_sorted_steps(e);
-    uint32_t age = e->sorted ? (uint32_t)(e->steps_done - e->sorted_since) : 0u;
+    const bool sorting = sorts_itself(e, n);
     while (n > 0) {
-        uint32_t m = n < kEnsChunk ? n : kEnsChunk;
+        uint32_t m = ens_chunk_of(e, n, sorting);
         if (e->reorder_every) {
             uint64_t to_next = e->reorder_every - steps % e->reorder_every;
             if (to_next < m) m = (uint32_t)to_next;
-        } else if (e->auto_sort && (e->sorted || e->unsorted_steps + n >= sorted_min_steps(agents))) {
-            if (age >= aged) age = 0;
-            if (aged - age < m) m = aged - age;
-            age += m;
         }
         if (!chunk_graph(e, m)) break; // stepping will launch directly
         if (m & 1) e->cur = 1 - e->cur;
@@ -825,7 +831,7 @@ int prepare_ens_steps(slime_ensemble* e, uint32_t n) {
 
 int run_ens_steps(slime_ensemble* e, uint32_t n) {
     while (n > 0) {
-        uint32_t m = n < kEnsChunk ? n : kEnsChunk;
+        uint32_t m = ens_chunk_of(e, n, sorts_itself(e, n));
         if (e->reorder_every) {
             if (e->steps_done % e->reorder_every == 0 && e->last_reorder_step != e->steps_done) {
                 int rc = reorder_all(e);
@@ -839,12 +845,8 @@ int run_ens_steps(slime_ensemble* e, uint32_t n) {
             int rc = ensure_lanes(e);
             if (rc != SLIME_OK) return rc;
         }
-        int rc = auto_sort(e, n);
+        int rc = auto_sort(e, n, m);
         if (rc != SLIME_OK) return rc;
-        if (e->sorted && e->auto_sort && !e->reorder_every) {
-            const uint64_t left = ens_sorted_steps(e) - (e->steps_done - e->sorted_since);
-            if (left < m) m = (uint32_t)left;
-        }
         rc = prepare_ens_deposits(e);
         if (rc != SLIME_OK) return rc;
         const uint64_t kernels = lanes ? m * lane_kernels_per_step(e) : m;

@@ -679,12 +679,36 @@ int do_reorder(slime_ctx* ctx) {
 // 251 / 276, 16 250 / 236, 100 250 / 212.  Hence:
 uint32_t sorted_min_steps(uint64_t n) { return n >= 200000 ? 16u : (n >= 32768 ? 64u : ~0u); }
 
+// The most cells an agent crosses in a step.
+float cells_a_step(const DevParams& d) {
+    const float lo = fabsf(d.speed_min), hi = fabsf(d.speed_max);
+    return (lo > hi ? lo : hi) * fabsf(d.time_step);
+}
+
+// Whether agents this fast, n in all, are sorted: fast ones lose the order in the
+// 16 steps between two sorts, and few ones gain less than the sort takes.
+// Measured, us a step in slot order / sorted, by the cells a step that the
+// fastest cross, on either side of each line:
+//   32,768 on 512^2 0.7 6.0 / 5.9, 1 6.0 / 6.1; 65,536 on 512^2 0.7 6.9 / 6.6, 1 6.8 /
+//     7.0, 2 7.0 / 8.1;
+//   131,072 on 512^2 1 7.6 / 7.4, 2 8.1 / 8.8, on 1024^2 1 8.3 / 7.6, 2 8.4 / 8.6;
+//   200,000 on 512^2 8 10.2 / 10.1, 16 9.8 / 11.2, on 1024^2 8 13.7 / 13.0, 16 13.9 /
+//     14.7; 400,000 on 1024^2 8 17.9 / 16.8, 16 17.3 / 19.7;
+//   1 M on 1024^2 24 32.6 / 32.3, 48 32.6 / 34.1; 2 M on 2048^2 24 62.3 / 60.7, 48 62.4 /
+//     64.5; 10 M on 1600x900 24 263 / 252, 48 263 / 269;
+//   on 4096^2, which such agents take long to cross, 1 M 128 70.2 / 66.5, 256 70.2 /
+//     69.9; 16.8 M 128 651 / 617, 256 651 / 670.
+bool sorting_pays(const DevParams& d, uint64_t n) {
+    const float most = n < 100000 ? 0.7f : (n < 200000 ? 1.0f : (n < 1000000 ? 8.0f
+                       : ((int64_t)d.W * d.H < 8000000 ? 24.0f : 128.0f)));
+    return cells_a_step(d) <= most;
+}
+
 // The copy is sorted again when the fastest agents have crossed 32 cells (100
 // steps of 10 M agents at 0.48 cells a step: 8 cells 151.7, 16 148.3, 32 146.5,
 // 64 149.8 us), at most every 16 steps.
 uint32_t sorted_steps_of(const DevParams& d) {
-    const float lo = fabsf(d.speed_min), hi = fabsf(d.speed_max);
-    const float move = (lo > hi ? lo : hi) * fabsf(d.time_step); // cells a step
+    const float move = cells_a_step(d);
     return move >= 2.0f ? 16u : (move > 0.032f ? (uint32_t)(32.0f / move) : 1000u);
 }
 
@@ -706,7 +730,7 @@ bool sorted_run_ready(slime_ctx* ctx, uint32_t n_steps) {
     const uint64_t n = ctx->agents.n, n_pad = ctx->agents.n_pad;
     if (ctx->opt.reorder_every || ctx->agents.ids || ctx->sorted_refused ||
         (uint64_t)n_steps + ctx->slot_steps < sorted_min_steps(n) ||
-        ctx->dev.dispatch_mode != SLIME_DISPATCH_EACH_AGENT)
+        ctx->dev.dispatch_mode != SLIME_DISPATCH_EACH_AGENT || !sorting_pays(ctx->dev, n))
         return false;
     if (!ctx->sorted_block) {
         const size_t bytes = 5 * n_pad * sizeof(float);
@@ -725,9 +749,10 @@ bool sorted_run_ready(slime_ctx* ctx, uint32_t n_steps) {
     return true;
 }
 
-// Before n_steps steps: onto the copy where that pays.
+// Before n_steps steps: onto the copy where that pays, and off it where the
+// agents have become too fast.
 int begin_sorted_run(slime_ctx* ctx, uint32_t n_steps) {
-    if (ctx->in_sorted_run) return SLIME_OK;
+    if (ctx->in_sorted_run) return sorting_pays(ctx->dev, ctx->agents.n) ? SLIME_OK : end_sorted_run(ctx);
     if (!sorted_run_ready(ctx, n_steps)) return SLIME_OK;
     AgentsSoA to = ctx->agents;
     to.x = (float*)ctx->sorted_block;

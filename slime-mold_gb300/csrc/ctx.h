@@ -162,6 +162,7 @@ void release_sorted(slime_ctx* ctx);
 cudaError_t ctx_alloc(slime_ctx* ctx, void** p, size_t bytes);
 // How many steps a sort of n agents is worth, and after how many it is done again.
 uint32_t sorted_min_steps(uint64_t n);
+bool sorting_pays(const DevParams& d, uint64_t n);
 uint32_t sorted_steps_of(const DevParams& d);
 uint32_t sorted_steps(const slime_ctx* ctx);
 int prepare_steps(slime_ctx* ctx, uint32_t n);

@@ -74,6 +74,7 @@ struct Colony {
     bool counts_dirty[2] = {false, false};
     bool marks_dirty[2] = {false, false};
     bool marks = false;
+    bool sorts = false; // by itself, without a schedule (update_sorts)
 };
 
 // Bounded grid barrier: every block arrives once; the last one to arrive
@@ -274,7 +275,7 @@ struct slime_ensemble {
     int device = 0;
     cudaStream_t stream = nullptr;
     std::vector<Colony> colonies;
-    uint64_t total_slots = 0, total_cells = 0;
+    uint64_t total_slots = 0, total_cells = 0, total_agents = 0;
     float* agent_block = nullptr; // x | y | angle | speed, total_slots each
     uint32_t* ids = nullptr;      // slot -> colony-local agent id (identity until reordered)
     uint32_t* check_flag = nullptr; // of uploaded trails
@@ -287,6 +288,8 @@ struct slime_ensemble {
     bool auto_sort = true;
     bool sorted = false;         // since the last upload or seed
     uint64_t unsorted_steps = 0; // steps made without
+    uint64_t sortable = 0;       // agents of the colonies that sort by themselves
+    uint32_t sorted_steps = 0;   // how long they stay in order
     uint64_t sorted_since = 0;   // steps_done at the last sort
     ReorderScratch reorder;
     ReorderScratch lane_reorder[3]; // sort scratch of the lanes engine's concurrent reorders (with `reorder`)
@@ -341,6 +344,21 @@ int ens_fail(slime_ensemble* e, int code, const char* msg) {
 void ens_invalidate(slime_ensemble* e) {
     for (auto& kv : e->graphs) cudaGraphExecDestroy(kv.second);
     e->graphs.clear();
+}
+
+// Which colonies a sort that no schedule asks for takes: those that launch_reorder
+// can sort and for which it pays (sorting_pays in capi.cu, on the agents of all);
+// and after how many steps: when the fastest agents of any have crossed 32 cells.
+void update_sorts(slime_ensemble* e) {
+    e->sortable = 0;
+    e->sorted_steps = 1000;
+    for (Colony& c : e->colonies) {
+        c.sorts = c.n > 0 && reorder_scratch_bytes(c.n, c.W, c.H, e->reorder_cell_log2) > 0 &&
+                  sorting_pays(c.dev, e->total_agents);
+        if (!c.sorts) continue;
+        e->sortable += c.n;
+        e->sorted_steps = std::min(e->sorted_steps, sorted_steps_of(c.dev));
+    }
 }
 
 int upload_cols(slime_ensemble* e) {
@@ -558,19 +576,15 @@ cudaError_t enqueue_lane_steps(slime_ensemble* e, uint32_t m) {
     return ce;
 }
 
-bool reorder_fits(const slime_ensemble* e, const Colony& c) {
-    return c.n > 0 && reorder_scratch_bytes(c.n, c.W, c.H, e->reorder_cell_log2) > 0;
-}
-
 // Morton-reorder every colony's slots (results are unchanged: each slot keeps
 // its colony-local id).  With the lanes engine's lanes in place the colonies'
 // sorts run on four of them at once (largest first, each onto the lane with
 // the fewest agents so far), each of those lanes with its own sort scratch;
 // otherwise one after another on the ensemble's stream.  With `fitting` only
-// the colonies that launch_reorder takes (reorder_fits).
+// the colonies that sort by themselves.
 int reorder_all(slime_ensemble* e, bool fitting = false) {
     auto sorts = [&](const Colony& c) {
-        return c.n > 0 && (!fitting || reorder_fits(e, c));
+        return c.n > 0 && (!fitting || c.sorts);
     };
     const size_t nr = e->lanes.size() < 4 ? e->lanes.size() : 4;
     cudaError_t ce = cudaSuccess;
@@ -612,30 +626,13 @@ int reorder_all(slime_ensemble* e, bool fitting = false) {
     return SLIME_OK;
 }
 
-// The agents of the colonies that can be sorted.
-uint64_t sortable_agents(const slime_ensemble* e) {
-    uint64_t n = 0;
-    for (const Colony& c : e->colonies)
-        if (reorder_fits(e, c)) n += c.n;
-    return n;
-}
-
-// Steps after which the colonies are sorted again when no schedule says so: when
-// the fastest agents of any have crossed 32 cells.
-uint32_t ens_sorted_steps(const slime_ensemble* e) {
-    uint32_t steps = 1000;
-    for (const Colony& c : e->colonies)
-        if (c.n) steps = std::min(steps, sorted_steps_of(c.dev));
-    return steps;
-}
-
 // Whether the scratch of a sort that no schedule asks for is there, or can come
 // from memory that is amply there (a quarter of what is free).  A lane's scratch
 // is its largest colony's, so the largest colonies' are what four lanes take.
 bool scratch_ready(const slime_ensemble* e) {
     std::vector<size_t> need;
     for (const Colony& c : e->colonies)
-        if (reorder_fits(e, c)) need.push_back(reorder_scratch_bytes(c.n, c.W, c.H, e->reorder_cell_log2));
+        if (c.sorts) need.push_back(reorder_scratch_bytes(c.n, c.W, c.H, e->reorder_cell_log2));
     std::sort(need.begin(), need.end(), std::greater<size_t>());
     const size_t nr = e->engine == SLIME_ENSEMBLE_LANES && e->lanes.size() > 1 ? std::min<size_t>(e->lanes.size(), 4) : 1;
     size_t more = 0;
@@ -663,14 +660,14 @@ void give_up_auto_sort(slime_ensemble* e) {
 // order).
 bool sorts_itself(const slime_ensemble* e, uint32_t n) {
     return !e->reorder_every && e->auto_sort &&
-           (e->sorted || (uint64_t)n + e->unsorted_steps >= sorted_min_steps(sortable_agents(e)));
+           (e->sorted || (uint64_t)n + e->unsorted_steps >= sorted_min_steps(e->sortable));
 }
 
 constexpr uint32_t kEnsChunk = 50;
 
 // How many of the next n steps are made at once (chunk_of in capi.cu).
 uint32_t ens_chunk_of(const slime_ensemble* e, uint32_t n, bool sorting) {
-    if (sorting) n = std::min(n, ens_sorted_steps(e));
+    if (sorting) n = std::min(n, e->sorted_steps);
     return std::min(n, kEnsChunk);
 }
 
@@ -678,7 +675,7 @@ uint32_t ens_chunk_of(const slime_ensemble* e, uint32_t n, bool sorting) {
 // when their order has aged.  Without scratch memory it is given up.
 int auto_sort(slime_ensemble* e, uint32_t n, uint32_t take) {
     if (!sorts_itself(e, n)) return SLIME_OK;
-    if (e->sorted && !resort_due(e->steps_done - e->sorted_since, take, ens_sorted_steps(e))) return SLIME_OK;
+    if (e->sorted && !resort_due(e->steps_done - e->sorted_since, take, e->sorted_steps)) return SLIME_OK;
     const int rc = scratch_ready(e) ? reorder_all(e, true) : SLIME_ERR_OUT_OF_MEMORY;
     if (rc == SLIME_ERR_OUT_OF_MEMORY) {
         give_up_auto_sort(e);
@@ -944,6 +941,7 @@ slime_ensemble* slime_ensemble_create(uint32_t k, const uint32_t* widths, const 
         c.trail_off = cells;
         slots += c.n_pad;
         cells += (uint64_t)c.W * c.H;
+        e->total_agents += c.n;
         // every colony's first cell 256-byte aligned (float4 rows, and a
         // base its gather texture accepts)
         cells = (cells + 63) & ~63ull;
@@ -989,6 +987,7 @@ slime_ensemble* slime_ensemble_create(uint32_t k, const uint32_t* widths, const 
         Colony& c = e->colonies[j];
         for (int i = 0; i < 2; i++) c.tex[i] = make_trail_texture(e->trail[i] + c.trail_off, c.W, c.H);
     }
+    update_sorts(e);
     if (rc == SLIME_OK) rc = upload_cols(e);
     if (rc == SLIME_OK) rc = build_agent_items(e);
     if (rc == SLIME_OK) rc = build_strip_items(e);
@@ -1045,6 +1044,7 @@ int slime_ensemble_set_params(slime_ensemble* e, uint32_t j, const SlimeParams* 
     c.params.width = c.W;
     c.params.height = c.H;
     c.dev = d;
+    update_sorts(e);
     // the cooperative kernel reads the colony table (its graphs stay valid);
     // the lanes engine's graphs hold the parameters as kernel arguments
     if (e->engine == SLIME_ENSEMBLE_LANES) {
@@ -1115,6 +1115,7 @@ int slime_ensemble_set_reorder(slime_ensemble* e, uint32_t every, uint32_t cell_
     e->reorder_every = every;
     unsorted(e);
     e->reorder_cell_log2 = (int)cell_log2;
+    update_sorts(e);
     return SLIME_OK;
 }
 
@@ -1254,7 +1255,7 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
         cudaMemcpyAsync(s + abytes + 2 * tbytes + i * tbytes, e->counts[i], tbytes, cudaMemcpyDeviceToDevice,
                         e->stream);
     }
-    if (e->reorder_every || (e->auto_sort && sorted_min_steps(sortable_agents(e)) < 1000)) { // as the steps will have them
+    if (e->reorder_every || (e->auto_sort && sorted_min_steps(e->sortable) < 1000)) { // as the steps will have them
         int rrc = e->reorder_every ? reorder_all(e) : (scratch_ready(e) ? reorder_all(e, true) : SLIME_ERR_OUT_OF_MEMORY);
         if (rrc == SLIME_OK && !e->reorder_every) {
             e->sorted = true;

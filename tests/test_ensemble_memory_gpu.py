@@ -31,7 +31,7 @@ def capped(code, cap, timeout=120):
     return out.stdout
 
 
-K, SIDE, N = 4, 64, 40_000  # colonies sorted every 16 steps: their fastest agents cross 2 cells a step
+K, SIDE, N = 4, 64, 60_000  # colonies sorted every 16 steps: their fastest agents cross 2 cells a step
 
 
 def params(j):
@@ -84,7 +84,7 @@ def test_colonies_too_wide_to_sort_step(gpu, engine, tuned):
     its agents come, the others of the ensemble are sorted.  By a schedule it
     is still refused."""
     import slime_gb300 as sg
-    sizes = [(262_148, 8, 40_000), (128, 96, 30_000)]
+    sizes = [(262_148, 8, 150_000), (128, 96, 210_000)]
     params = [config0_params(W, H, agent_speed_min=60.0, agent_speed_max=125.0) for W, H, _ in sizes]
     ens = sg.Ensemble([s[0] for s in sizes], [s[1] for s in sizes], [s[2] for s in sizes], params)
     ens.set_engine(engine)

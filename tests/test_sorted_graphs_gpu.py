@@ -17,7 +17,7 @@ import sys
 sys.path.insert(0, %r); sys.path.insert(0, %r)
 import slime_gb300 as sg
 from conftest import agents_uniform, config0_params
-W, H, n = 256, 192, 40_000
+W, H, n = 256, 192, 200_003
 p = config0_params(W, H, agent_speed_min=20.0, agent_speed_max=43.75)  # 0.7 cells a step: sorted every 45 steps
 agents = agents_uniform(n, W, H, 20.0, 43.75, seed=1)
 """ % (os.path.join(ROOT, "slime-mold_gb300"), os.path.join(ROOT, "tests"))
@@ -29,7 +29,7 @@ def child(code, graphs):
     assert out.returncode == 0, out.stdout + out.stderr
 
 
-# calls of 100: chunks of 45, 45 and 10 from either buffer; single steps: 64 in
+# calls of 100: chunks of 45, 45 and 10 from either buffer; single steps: 15 in
 # slot order and the rest on the copy, from either buffer
 @pytest.mark.parametrize("calls,steps,graphs", [(25, 100, 4), (300, 1, 4), (40, 7, 4)])
 def test_contexts(gpu, calls, steps, graphs):

@@ -69,7 +69,7 @@ np.savez({str(tmp_path / "out.npz")!r}, **out)
 
 def test_ensemble_of_thin_colonies(gpu, tmp_path):
     import slime_gb300 as sg
-    sizes = [(65_536, 16, 60_000), (131_076, 8, 50_000)]
+    sizes = [(65_536, 16, 120_000), (131_076, 8, 100_000)]
     code = f"""
 sizes = {sizes}
 ens = sg.Ensemble([s[0] for s in sizes], [s[1] for s in sizes], [s[2] for s in sizes],

@@ -366,7 +366,10 @@ int slime_ensemble_autotune(slime_ensemble* ens, uint32_t reps);
  *   agents, a bounded grid barrier, all colonies' trail strips);
  * LANES - each colony's steps as a chain of the single-colony kernels on one
  *   of up to 64 lanes forked from the ensemble's stream, one CUDA graph per
- *   chunk of steps, so that the colonies' chains run concurrently. */
+ *   chunk of steps, so that the colonies' chains run concurrently.
+ * An ensemble of up to 64 colonies that was neither tuned nor told takes LANES for
+ * calls of several steps or large colonies, from the second call with the same
+ * parameters on, and COOPERATIVE for the others. */
 #define SLIME_ENSEMBLE_COOPERATIVE 0u
 #define SLIME_ENSEMBLE_LANES 1u
 /* Choose the engine by hand; for LANES also the agent-kernel shape and trail
@@ -398,7 +401,7 @@ typedef struct SlimeEnsembleInfo {
     uint32_t strip_rows;    /* trail rows per strip work item (autotuned) */
     uint32_t agents_per_thread; /* cooperative engine: agents a thread steps per agent work item, 4
                                    (each alone) or 2 (as one pair); autotuned */
-    uint32_t engine;            /* SLIME_ENSEMBLE_COOPERATIVE or SLIME_ENSEMBLE_LANES */
+    uint32_t engine;            /* SLIME_ENSEMBLE_COOPERATIVE or SLIME_ENSEMBLE_LANES: of the last steps */
     uint32_t lanes;             /* capture lanes of the lanes engine (0 until it first steps) */
     uint32_t lane_agent_shape;  /* lanes engine: agent-kernel shape (slime_set_agent_shape's table) */
     uint32_t lane_trail_tile;   /* lanes engine: trail tile (slime_set_trail_tile's table) */

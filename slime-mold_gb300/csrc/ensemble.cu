@@ -288,6 +288,7 @@ struct slime_ensemble {
     bool auto_sort = true;
     bool sorted = false;         // since the last upload or seed
     uint64_t unsorted_steps = 0; // steps made without
+    bool sorts_stale = true;     // update_sorts is due
     uint64_t sortable = 0;       // agents of the colonies that sort by themselves
     uint32_t sorted_steps = 0;   // how long they stay in order
     uint64_t sorted_since = 0;   // steps_done at the last sort
@@ -315,7 +316,8 @@ struct slime_ensemble {
     bool use_graphs = true;
     bool last_chunk_graph = false; // the last chunk of steps replayed a graph
     int engine = SLIME_ENSEMBLE_COOPERATIVE;
-    bool engine_chosen = false; // by hand, by its shape or by the autotuner
+    bool engine_chosen = false; // by hand, by its shape or by the autotuner; else pick_engine
+    uint64_t stable_steps = 0;  // steps made since parameters were set
     int lane_agent_shape = 13; // agent-kernel shape of the lanes engine (persistent, texture gather)
     int lane_trail_tile = 8;   // trail tile of the lanes engine (streaming, 16-row strips)
     int max_lanes = 0;         // lanes of the lanes engine (0: one per colony, at most 64)
@@ -346,10 +348,28 @@ void ens_invalidate(slime_ensemble* e) {
     e->graphs.clear();
 }
 
+// The lanes engine's graphs, which hold parameters and record kinds.
+constexpr int kLaneGraph = 2; // bit of the key's second number, beside the parity
+void drop_lane_graphs(slime_ensemble* e) {
+    bool any = false;
+    for (const auto& kv : e->graphs) any = any || (kv.first.second & kLaneGraph);
+    if (any) cudaStreamSynchronize(e->stream);
+    for (auto it = e->graphs.begin(); it != e->graphs.end();) {
+        if (it->first.second & kLaneGraph) {
+            cudaGraphExecDestroy(it->second);
+            it = e->graphs.erase(it);
+        } else {
+            ++it;
+        }
+    }
+}
+
 // Which colonies a sort that no schedule asks for takes: those that launch_reorder
 // can sort and for which it pays (sorting_pays in capi.cu, on the agents of all);
 // and after how many steps: when the fastest agents of any have crossed 32 cells.
 void update_sorts(slime_ensemble* e) {
+    if (!e->sorts_stale) return;
+    e->sorts_stale = false;
     e->sortable = 0;
     e->sorted_steps = 1000;
     for (Colony& c : e->colonies) {
@@ -708,6 +728,9 @@ bool colony_marks(const slime_ensemble* e, const Colony& c) {
            c.trail_clean && c.dev.dep >= 1.0f && keeps_trail_clean(c.dev) && trail_tile_streams(c.dev, e->lane_trail_tile);
 }
 
+// Whether the steps of the current engine record c's deposits as marks.
+bool records_marks(const slime_ensemble* e, const Colony& c) { return e->engine == SLIME_ENSEMBLE_LANES && c.marks; }
+
 // Both mark arrays, or none: without memory for them the colonies count.
 void alloc_marks(slime_ensemble* e) {
     cudaError_t ce = cudaSuccess;
@@ -725,8 +748,8 @@ void alloc_marks(slime_ensemble* e) {
     e->marks_refused = true;
 }
 
-// Before a chunk: each colony's record kind (a change drops the captured
-// graphs, which hold it), and the record the chunk's first step writes
+// Before a chunk: in the lanes engine each colony's record kind (a change drops the
+// captured graphs, which hold it), and the record the chunk's first step writes
 // (counts[cur] or marks[cur]) cleared where steps of the other kind or the
 // other engine left deposits in it.
 int prepare_ens_deposits(slime_ensemble* e) {
@@ -734,15 +757,16 @@ int prepare_ens_deposits(slime_ensemble* e) {
     for (const Colony& c : e->colonies)
         if (!e->marks[0] && colony_marks(e, c)) alloc_marks(e);
     for (Colony& c : e->colonies) {
+        if (e->engine != SLIME_ENSEMBLE_LANES) break;
         const bool mk = colony_marks(e, c);
         changed = changed || mk != c.marks;
         c.marks = mk;
     }
-    if (changed) ens_invalidate(e);
+    if (changed) drop_lane_graphs(e);
     const int cur = e->cur;
     for (Colony& c : e->colonies) {
         const size_t cells = (size_t)c.W * c.H;
-        if (c.marks) {
+        if (records_marks(e, c)) {
             if (c.marks_dirty[cur]) {
                 ECK(cudaMemsetAsync(e->marks[cur] + c.trail_off, 0, cells, e->stream), "clearing deposit marks");
                 c.marks_dirty[cur] = false;
@@ -761,7 +785,7 @@ int prepare_ens_deposits(slime_ensemble* e) {
 void after_ens_steps(slime_ensemble* e, uint32_t m) {
     if (m == 0) return;
     for (Colony& c : e->colonies) {
-        bool* dirty = c.marks ? c.marks_dirty : c.counts_dirty;
+        bool* dirty = records_marks(e, c) ? c.marks_dirty : c.counts_dirty;
         dirty[e->cur] = false;
         dirty[1 - e->cur] = true;
         c.trail_clean = c.trail_clean && keeps_trail_clean(c.dev);
@@ -772,7 +796,7 @@ void after_ens_steps(slime_ensemble* e, uint32_t m) {
 // captured on first use; null when the capture fails (the caller then
 // launches directly).
 cudaGraphExec_t chunk_graph(slime_ensemble* e, uint32_t m) {
-    auto key = std::make_pair(m, e->cur);
+    auto key = std::make_pair(m, e->cur | (e->engine == SLIME_ENSEMBLE_LANES ? kLaneGraph : 0));
     auto it = e->graphs.find(key);
     if (it != e->graphs.end()) return it->second;
     const int saved = e->cur;
@@ -796,26 +820,47 @@ cudaGraphExec_t chunk_graph(slime_ensemble* e, uint32_t m) {
     return exec;
 }
 
+// The engine of the next m steps where none was chosen or tuned.  Lanes take a
+// launch per colony and pass in every chunk, and their graphs are captured anew
+// when a parameter changes; the cooperative kernel takes one launch a step and
+// reads the parameters.  Microseconds a step, cooperative / lanes, half an agent a
+// cell: 4 colonies of 256^2 45 / 21 in calls of one step and 41 / 12 of ten; 16 of
+// 256^2 49 / 79 and 44 / 20; 16 of 512^2 94 / 92 and 89 / 38; 48 of 128^2 45 / 283 and
+// 41 / 45.  With every parameter set before each call: 16 of 256^2 208 / 398 and
+// 60 / 130, 48 of 128^2 554 / 1219 and 91 / 364.  Hence lanes for four steps a colony
+// and more at once or colonies of 100,000 agents and quarter cells on average, and
+// only where as many steps were made with these parameters before or the
+// graph is there.
+void pick_engine(slime_ensemble* e, uint32_t m, bool prepared) {
+    const uint64_t k = e->colonies.size();
+    if (e->engine_chosen || k > kMaxLanes) return;
+    const bool pays = 4 * (uint64_t)m >= k || e->total_agents + e->total_cells / 4 >= 100000 * k;
+    const bool there = prepared || e->stable_steps >= m || e->graphs.count({m, e->cur | kLaneGraph});
+    e->engine = pays && there ? SLIME_ENSEMBLE_LANES : SLIME_ENSEMBLE_COOPERATIVE;
+}
+
 // Capture the graphs that the next n steps replay (run_ens_steps' chunks).
 int prepare_ens_steps(slime_ensemble* e, uint32_t n) {
-    const bool lanes = e->engine == SLIME_ENSEMBLE_LANES;
-    if (!e->use_graphs && !lanes) return SLIME_OK;
-    if (lanes) {
-        int rc = ensure_lanes(e);
-        if (rc != SLIME_OK) return rc;
-    }
-    // the record kinds the graphs hold (clearing a stale record early is
-    // what the next step would do first)
-    int rc = prepare_ens_deposits(e);
-    if (rc != SLIME_OK) return rc;
     const int saved = e->cur;
     uint64_t steps = e->steps_done;
+    update_sorts(e);
     const bool sorting = sorts_itself(e, n);
     while (n > 0) {
         uint32_t m = ens_chunk_of(e, n, sorting);
         if (e->reorder_every) {
             uint64_t to_next = e->reorder_every - steps % e->reorder_every;
             if (to_next < m) m = (uint32_t)to_next;
+        }
+        pick_engine(e, m, true);
+        const bool lanes = e->engine == SLIME_ENSEMBLE_LANES;
+        if (!e->use_graphs && !lanes) break;
+        int rc = lanes ? ensure_lanes(e) : SLIME_OK;
+        // the record kinds the graphs hold (clearing a stale record early is
+        // what the next step would do first)
+        if (rc == SLIME_OK && steps == e->steps_done) rc = prepare_ens_deposits(e);
+        if (rc != SLIME_OK) {
+            e->cur = saved;
+            return rc;
         }
         if (!chunk_graph(e, m)) break; // stepping will launch directly
         if (m & 1) e->cur = 1 - e->cur;
@@ -827,6 +872,7 @@ int prepare_ens_steps(slime_ensemble* e, uint32_t n) {
 }
 
 int run_ens_steps(slime_ensemble* e, uint32_t n) {
+    update_sorts(e);
     while (n > 0) {
         uint32_t m = ens_chunk_of(e, n, sorts_itself(e, n));
         if (e->reorder_every) {
@@ -837,6 +883,7 @@ int run_ens_steps(slime_ensemble* e, uint32_t n) {
             uint64_t to_next = e->reorder_every - e->steps_done % e->reorder_every;
             if (to_next < m) m = (uint32_t)to_next;
         }
+        pick_engine(e, m, false);
         const bool lanes = e->engine == SLIME_ENSEMBLE_LANES;
         if (lanes) {
             int rc = ensure_lanes(e);
@@ -864,6 +911,7 @@ int run_ens_steps(slime_ensemble* e, uint32_t n) {
         after_ens_steps(e, m);
         e->launches += kernels;
         e->steps_done += m;
+        e->stable_steps += m;
         if (!e->sorted) e->unsorted_steps += m;
         n -= m;
     }
@@ -987,15 +1035,12 @@ slime_ensemble* slime_ensemble_create(uint32_t k, const uint32_t* widths, const 
         Colony& c = e->colonies[j];
         for (int i = 0; i < 2; i++) c.tex[i] = make_trail_texture(e->trail[i] + c.trail_off, c.W, c.H);
     }
-    update_sorts(e);
     if (rc == SLIME_OK) rc = upload_cols(e);
     if (rc == SLIME_OK) rc = build_agent_items(e);
     if (rc == SLIME_OK) rc = build_strip_items(e);
     if (rc == SLIME_OK) rc = size_grid(e);
-    // Untuned: the lanes for up to as many colonies as there are lanes (16 colonies
-    // of 256^2 to 1024^2, in no order: 543 us a step against 584), the one
-    // launch per step for more, whose captured chains would be that many times
-    // as many nodes.
+    // Untuned, with no more colonies than lanes: pick_engine; the lanes are what it
+    // comes to.
     if (k <= kMaxLanes) e->engine = SLIME_ENSEMBLE_LANES;
     if (rc != SLIME_OK) {
         *status = rc;
@@ -1044,13 +1089,11 @@ int slime_ensemble_set_params(slime_ensemble* e, uint32_t j, const SlimeParams* 
     c.params.width = c.W;
     c.params.height = c.H;
     c.dev = d;
-    update_sorts(e);
+    e->sorts_stale = true;
     // the cooperative kernel reads the colony table (its graphs stay valid);
     // the lanes engine's graphs hold the parameters as kernel arguments
-    if (e->engine == SLIME_ENSEMBLE_LANES) {
-        cudaStreamSynchronize(e->stream);
-        ens_invalidate(e);
-    }
+    drop_lane_graphs(e);
+    e->stable_steps = 0;
     return upload_cols(e);
 }
 
@@ -1115,7 +1158,7 @@ int slime_ensemble_set_reorder(slime_ensemble* e, uint32_t every, uint32_t cell_
     e->reorder_every = every;
     unsorted(e);
     e->reorder_cell_log2 = (int)cell_log2;
-    update_sorts(e);
+    e->sorts_stale = true;
     return SLIME_OK;
 }
 
@@ -1255,6 +1298,7 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
         cudaMemcpyAsync(s + abytes + 2 * tbytes + i * tbytes, e->counts[i], tbytes, cudaMemcpyDeviceToDevice,
                         e->stream);
     }
+    update_sorts(e);
     if (e->reorder_every || (e->auto_sort && sorted_min_steps(e->sortable) < 1000)) { // as the steps will have them
         int rrc = e->reorder_every ? reorder_all(e) : (scratch_ready(e) ? reorder_all(e, true) : SLIME_ERR_OUT_OF_MEMORY);
         if (rrc == SLIME_OK && !e->reorder_every) {
@@ -1308,6 +1352,7 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
         return check_barrier(e);
     };
     // cooperative engine: agents per thread x strip rows x residency
+    e->engine_chosen = true;
     e->engine = SLIME_ENSEMBLE_COOPERATIVE;
     for (int ao : apt_opts) {
       e->apt = ao;
@@ -1386,7 +1431,6 @@ int slime_ensemble_autotune(slime_ensemble* e, uint32_t reps) {
     e->blocks_per_sm = best_bps;
     e->apt = best_apt;
     e->engine = best_engine;
-    e->engine_chosen = true;
     e->lane_agent_shape = best_shape;
     e->lane_trail_tile = best_tile;
     ens_invalidate(e);
@@ -1441,7 +1485,7 @@ int slime_ensemble_get_info(const slime_ensemble* e, SlimeEnsembleInfo* out) {
     out->lanes = (uint32_t)e->lanes.size();
     out->lane_agent_shape = (uint32_t)e->lane_agent_shape;
     out->lane_trail_tile = (uint32_t)e->lane_trail_tile;
-    for (const Colony& c : e->colonies) out->marks_colonies += c.marks ? 1u : 0u;
+    for (const Colony& c : e->colonies) out->marks_colonies += records_marks(e, c) ? 1u : 0u;
     return SLIME_OK;
 }
 

@@ -120,8 +120,8 @@ def test_steps_without_memory_for_marks(gpu, tmp_path, spare):
 S, n = {side}, {n}
 ens = sg.Ensemble([S], [S], [n], [config0_params(S, S)])
 ens.upload_agents(0, agents_uniform(n, S, S, 1.0, 2.0, seed=1))
-ens.step(3)
-ens.step(20)
+for m in (3, 20, 20):  # calls of a length run on lanes from the second
+    ens.step(m)
 np.savez({str(tmp_path / "out.npz")!r}, a=ens.download_agents(0), t=ens.download_trail(0),
          marks=ens.info().marks_colonies, engine=ens.info().engine)
 """
@@ -130,6 +130,6 @@ np.savez({str(tmp_path / "out.npz")!r}, a=ens.download_agents(0), t=ens.download
     assert got["engine"] == sg.ENSEMBLE_LANES and got["marks"] == 0
     with sg.Simulation(side, side, n, config0_params(side, side)) as sim:
         sim.upload_agents(agents_uniform(n, side, side, 1.0, 2.0, seed=1))
-        sim.step(23)
+        sim.step(43)
         assert_bitexact(got["a"], sim.download_agents(), "agents")
         assert_bitexact(got["t"], sim.download_trail(), "trail")

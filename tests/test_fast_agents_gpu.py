@@ -55,6 +55,7 @@ def test_ensembles_sort_only_their_slow_colonies(gpu):
         agents = agents_uniform(n, W, H, 60.0, 900.0, seed=j)
         ens.upload_agents(j, agents)
         sim.upload_agents(agents)
+    ens.set_engine(sg.ENSEMBLE_LANES)
     before = ens.launch_count()
     ens.step(40)
     assert ens.launch_count() - before == 40 * 2 * 2 + 6 * 3  # the slow one's sorts, every 16 steps

@@ -47,6 +47,7 @@ def test_ensembles(gpu, calls, steps, graphs):
     child(f"""
 ens = sg.Ensemble([W], [H], [n], [p])
 ens.upload_agents(0, agents)
+ens.set_engine(sg.ENSEMBLE_LANES)
 for _ in range({calls}):
     ens.step({steps})
     assert ens.info().graphs_in_use == 1

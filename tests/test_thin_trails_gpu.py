@@ -76,6 +76,7 @@ ens = sg.Ensemble([s[0] for s in sizes], [s[1] for s in sizes], [s[2] for s in s
                   [config0_params(W, H, agent_speed_min=60.0, agent_speed_max=125.0) for W, H, n in sizes])
 for j, (W, H, n) in enumerate(sizes):
     ens.upload_agents(j, agents_uniform(n, W, H, 60.0, 125.0, seed=j))
+ens.set_engine(sg.ENSEMBLE_LANES)
 before = ens.launch_count()
 ens.step(70)
 np.savez({str(tmp_path / "out.npz")!r}, launches=ens.launch_count() - before,

@@ -668,9 +668,9 @@ int do_reorder(slime_ctx* ctx) {
 // So once enough steps are to be made, or were made one by one, the agents are
 // sorted into a copy that is stepped in their place (`agents`, with the id of
 // every slot) until something needs them in their slots: reordering by hand or
-// by schedule, the reference's dispatch, the autotuner, a resize.  Reading them
-// back does not (records go out in id order either way), and what replaces them
-// drops the copy.  The results are the same.
+// by schedule, the reference's dispatch, a resize.  Reading them back does not
+// (records go out in id order either way), the autotuner times its trials on the
+// copy, and what replaces the agents drops it.  The results are the same.
 // Measured (us a step, in slot order / on a copy, sort and return included): 65,536 agents on 512^2, 32
 // steps 6.5 / 6.9, 100 steps 6.5 / 6.1; 262,144 on 1024^2, 16 steps 13.0 / 11.7,
 // 100 12.8 / 9.0; 500,003 on 1001x777, 16 22.8 / 19.6, 100 22.6 / 17.6;
@@ -836,7 +836,7 @@ int tune_full_steps(slime_ctx* ctx, uint32_t steps, const int tiles[2]) {
     }
     const int cur = ctx->cur;
     auto restore = [&]() -> cudaError_t {
-        cudaError_t e = cudaMemcpyAsync(ctx->agent_block, snap, abytes, cudaMemcpyDeviceToDevice, ctx->stream);
+        cudaError_t e = cudaMemcpyAsync(ctx->agents.x, snap, abytes, cudaMemcpyDeviceToDevice, ctx->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(ctx->trail[cur], snap + abytes, tbytes, cudaMemcpyDeviceToDevice, ctx->stream);
         for (int i = 0; i < 2 && e == cudaSuccess; i++) {
@@ -849,7 +849,7 @@ int tune_full_steps(slime_ctx* ctx, uint32_t steps, const int tiles[2]) {
     };
     const bool marks = use_marks(ctx);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    cudaError_t e = cudaMemcpyAsync(snap, ctx->agent_block, abytes, cudaMemcpyDeviceToDevice, ctx->stream);
+    cudaError_t e = cudaMemcpyAsync(snap, ctx->agents.x, abytes, cudaMemcpyDeviceToDevice, ctx->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(snap + abytes, ctx->trail[cur], tbytes, cudaMemcpyDeviceToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaEventCreate(&e0);
@@ -1592,8 +1592,11 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
     if (!ctx) return SLIME_ERR_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
     if (reps == 0) reps = 5;
-    const int erc = end_sorted_run(ctx);
-    if (erc != SLIME_OK) return erc;
+    // the agents in the order that the steps will have them: on the copy where many
+    // steps would run on one
+    int src = begin_sorted_run(ctx, 1000);
+    if (src == SLIME_OK) src = resort_run(ctx, 50);
+    if (src != SLIME_OK) return src;
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0), "creating events");
     CK(cudaEventCreate(&e1), "creating events");
@@ -1638,7 +1641,7 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
     }
     // 2. agent-kernel shapes, on a snapshot of the agents that is put back
     // afterwards (the trial passes write agents and the deposit record).
-    // With reordering on, the agents are put in Morton order first, as the
+    // With a schedule, the agents are put in Morton order first, as the
     // steps will have them.  Each shape starts from the snapshot, makes one
     // untimed pass (the copy back evicts the trail from L2) and is timed over
     // `reps` passes in a row with the deposit record the steps will use; those
@@ -1653,7 +1656,7 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
         const size_t abytes = 4 * ctx->agents.n_pad * sizeof(float);
         void* snap = nullptr;
         if (dev_alloc((void**)&snap, abytes) == cudaSuccess) {
-            CK(cudaMemcpyAsync(snap, ctx->agent_block, abytes, cudaMemcpyDeviceToDevice, ctx->stream), "snapshot");
+            CK(cudaMemcpyAsync(snap, ctx->agents.x, abytes, cudaMemcpyDeviceToDevice, ctx->stream), "snapshot");
             float best_a = 1e30f;
             std::vector<float> first((size_t)agent_shape_count(), 0.0f);
             for (int round = 0; round < 2; round++)
@@ -1662,7 +1665,7 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
                     if (agent_shape_uses_texture(sh) && !ctx->trail_tex[cur]) continue;
                     // timed again only if it came near the best the first time
                     if (round == 1 && first[sh] > 1.1f * best_a) continue;
-                    cudaMemcpyAsync(ctx->agent_block, snap, abytes, cudaMemcpyDeviceToDevice, ctx->stream);
+                    cudaMemcpyAsync(ctx->agents.x, snap, abytes, cudaMemcpyDeviceToDevice, ctx->stream);
                     launch_agents(ctx->dev, ctx->agents, ctx->trail[cur], ctx->counts[cur], ctx->stream, sh, nullptr,
                                   ctx->trail_tex[cur], marks);
                     cudaEventRecord(e0, ctx->stream);
@@ -1680,7 +1683,7 @@ int slime_autotune(slime_ctx* ctx, uint32_t reps) {
                         best_shape = sh;
                     }
                 }
-            CK(cudaMemcpyAsync(ctx->agent_block, snap, abytes, cudaMemcpyDeviceToDevice, ctx->stream), "restore");
+            CK(cudaMemcpyAsync(ctx->agents.x, snap, abytes, cudaMemcpyDeviceToDevice, ctx->stream), "restore");
             CK(cudaMemsetAsync(ctx->counts[cur], 0, cells * sizeof(uint32_t), ctx->stream), "restore");
             if (mk) CK(cudaMemsetAsync(ctx->marks[cur], 0, cells, ctx->stream), "restore");
             CK(cudaStreamSynchronize(ctx->stream), "autotuning");

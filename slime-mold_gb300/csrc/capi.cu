@@ -354,10 +354,6 @@ cudaError_t ctx_alloc(slime_ctx* ctx, void** p, size_t bytes) {
     if (end_sorted_run(ctx) != SLIME_OK) return e;
     release_sorted(ctx);
     ctx->sorted_refused = true;
-    if (!ctx->agents.ids) {
-        dev_free(ctx->reorder.buf);
-        ctx->reorder = ReorderScratch();
-    }
     return dev_alloc(p, bytes);
 }
 
@@ -714,12 +710,17 @@ uint32_t sorted_steps_of(const DevParams& d) {
 
 uint32_t sorted_steps(const slime_ctx* ctx) { return sorted_steps_of(ctx->dev); }
 
+// Gives the copy back, which nothing steps any more, and the sort scratch with it
+// unless the context reorders its own agents.
 void release_sorted(slime_ctx* ctx) {
     if (!ctx->sorted_block) return;
     cudaStreamSynchronize(ctx->stream);
     invalidate_graphs(ctx);
     dev_free(ctx->sorted_block);
     ctx->sorted_block = nullptr;
+    if (ctx->agents.ids) return;
+    dev_free(ctx->reorder.buf);
+    ctx->reorder = ReorderScratch();
 }
 
 // Whether n_steps are run on a copy; allocates it on first use, only where it and

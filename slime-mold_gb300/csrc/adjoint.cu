@@ -739,6 +739,7 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
         const uint32_t m = (a.n_steps - s0) < K ? (a.n_steps - s0) : K;
         const bool held = a.seg_holds == (int)j;
         if (!held) { // replay the segment from its checkpoint, keeping T_s and k_s
+            a.seg_holds = -1; // until that is launched
             CK(cudaMemcpyAsync(a.agents_tmp, a.ckpt_agents + (size_t)j * 4 * a.n_pad, 4 * a.n_pad * sizeof(float),
                                cudaMemcpyDeviceToDevice, ctx->stream), "restoring agents");
             if (a.with_ids)
@@ -747,13 +748,13 @@ int slime_backward(slime_ctx* ctx, const float* dl_dtrail_final, SlimeGrads* gra
             CK(cudaMemcpyAsync(a.seg_trail, a.ckpt_trail + (size_t)j * cells, cells * sizeof(float),
                                cudaMemcpyDeviceToDevice, ctx->stream), "restoring trail");
             CK(cudaMemsetAsync(a.seg_counts, 0, (size_t)m * stride * sizeof(uint32_t), ctx->stream), "clearing counts");
-            a.seg_holds = (int)j;
         }
         cudaGraphExec_t exec = segment_graph(m, cg, held);
         if (exec)
             CK(cudaGraphLaunch(exec, ctx->stream), "launching a backward segment");
         else
             CK(enqueue_segment(m, cg, held), "replaying a segment and its backward steps");
+        a.seg_holds = (int)j;
         if (!held) ctx->launches += (uint64_t)m * agent_pass_kernels(a.dev, a.n, false) + (m - 1);
         ctx->launches += m;
         if (m & 1) cg = 1 - cg;

@@ -448,8 +448,8 @@ bool agent_shape_uses_texture(int i) { return i >= 12 && i <= 15; }
 
 // The persistent gathering shape (13) with a texture, and for many agents
 // without one (where it reads by pointer); one agent per thread (2) for fewer.
-// Steps in slot order / Morton order, us, shapes 0 (four agents per thread, the
-// default before) / 2 / 13: 10 M on 1600x900 314 / 314 / 271, 166 / 184 / 130;
+// Steps in slot order / Morton order, us, shapes 0 (four agents per
+// thread) / 2 / 13: 10 M on 1600x900 314 / 314 / 271, 166 / 184 / 130;
 // 65,536 on 512^2 10.3 / 7.4 / 7.4, 9.0 / 6.5 / 6.7; without a texture 500,003
 // on 1001x777 25.6 / 22.0 / 22.9, 18.0 / 16.2 / 16.4, 4 M on 3001x2003 148 /
 // 149 / 143, 89 / 93 / 87.

@@ -8,9 +8,9 @@ namespace {
 
 // A thread makes four pixels of a row, from a table of packed colours that the
 // block builds once in shared memory: one lookup and a quarter of a 16-byte
-// store a pixel instead of three byte loads and a 4-byte store.  Bound by the
-// two divisions a pixel and launch latency: a 1600x900 image of a 4096^2 trail
-// 6.0 us before and 4.6 now, a 1001x777 one of its own trail 4.3 and 3.2.
+// store a pixel.  Bound by the two divisions a pixel and launch latency: a
+// 1600x900 image of a 4096^2 trail 4.6 us, a 1001x777 one of its own trail 3.2 (6.0
+// and 4.3 with a pixel a thread, three byte loads and a 4-byte store each).
 __global__ void __launch_bounds__(256) colorize_kernel(const float* __restrict__ trail, int W, int H,
                                                        const uint8_t* __restrict__ lut, int tw, int th, float scale,
                                                        float off_x, float off_y, uint32_t* __restrict__ rgba,

@@ -73,7 +73,7 @@ struct slime_ctx {
 
     static constexpr int kGraphSorted = 4; // on the sorted copy
     static constexpr int kGraphRecord = 8; // the last segment of a recording
-    std::map<std::pair<uint32_t, int>, cudaGraphExec_t> graphs; // (steps, start parity | record << 1 | the two bits below) -> graph
+    std::map<std::pair<uint32_t, int>, cudaGraphExec_t> graphs; // (steps, start parity | marks << 1 | the two bits below) -> graph
 
     uint64_t steps_done = 0;
     uint64_t launches = 0;

@@ -56,10 +56,12 @@ cudaError_t launch_agents_caller(const DevParams& p, const AgentsSoA& a, const f
 int agent_pass_kernels(const DevParams& p, uint64_t n, bool marks);
 // How many agents (ids 0 .. this - 1) the reference's dispatch updates.
 uint64_t reference_dispatch_updated(uint64_t n);
-// Adds to `counts` the deposits the last step made, from the agents it left
-// (an agent deposits at the cell it moves to).
+// Whether a trail of this many cells is looked at on the device after an upload
+// (trail.cu), and that look: sets *flag where a value is negative or NaN.
 bool device_check_pays(uint64_t cells);
 cudaError_t launch_trail_check(const float* t, uint64_t n, uint32_t* flag, cudaStream_t s);
+// Adds to `counts` the deposits the last step made, from the agents it left
+// (an agent deposits at the cell it moves to).
 cudaError_t launch_recount(const DevParams& p, const AgentsSoA& a, uint32_t* counts, cudaStream_t s);
 cudaTextureObject_t make_trail_texture(const float* trail, uint32_t W, uint32_t H);
 // AoS staging (x, y, angle, speed per agent, id order) <-> SoA slots.

@@ -98,8 +98,6 @@ TrailTile trail_tile(int index) {
 //     1600x900 6.4 / 6.5, 2048^2 12.5 / 9.9;
 //   what strips cannot run, 4 / 5: radius 5 1600x900 7.5 / 7.3, 2048^2
 //     15.5 / 13.1; radius 1 3001x2003 18.9 / 20.9, radius 2 19.9 / 17.9.
-// (The 64 x 16 tile of one cell per thread that was the default before took
-// 6.6 and 14.4 for the two smallest boxes, 43.6 for radius 5 at 2048^2.)
 int trail_tile_default(const DevParams& p, bool marks, bool aligned) {
     const int64_t cells = (int64_t)p.W * p.H;
     const bool gauss = p.blur_mode == SLIME_BLUR_GAUSS;
@@ -122,7 +120,7 @@ bool trail_tile_streams(const DevParams& p, int tile) { return tile >= kNumTiles
 
 // Whether the values of an uploaded trail are looked at on the device, where
 // they just arrived, or by the host (which deposit marks want finite and >= 0,
-// or +inf).  An upload takes, host (scalar loop, the only one before; an OR
+// or +inf).  An upload takes, host (a scalar loop; an OR
 // over all values, which vectorises, takes 10 us less at 256^2) / device: 128^2
 // 15.5 / 28.7 us, 256^2 40.9 / 30.3, 512^2 117 / 35, 1024^2 431 / 53, 4096^2
 // 6689 / 423 (of which the copy takes all but 20).

@@ -268,7 +268,8 @@ int slime_set_steps_done(slime_ctx* ctx, uint64_t steps_done);
 int slime_step(slime_ctx* ctx, uint32_t n_steps);
 /* Capture now the CUDA graphs that the next n_steps steps will replay (the
  * same chunks slime_step cuts), without stepping: the first slime_step over
- * them then only replays.  Graphs stay valid until a parameter, option or
+ * them then only replays.  Where those steps would run on a sorted copy of the
+ * agents, the copy is made now.  Graphs stay valid until a parameter, option or
  * buffer change (or the first reorder, which adds the id buffer) drops them. */
 int slime_prepare_steps(slime_ctx* ctx, uint32_t n_steps);
 int slime_sync(slime_ctx* ctx);

@@ -369,8 +369,8 @@ int slime_ensemble_autotune(slime_ensemble* ens, uint32_t reps);
  *   of up to 64 lanes forked from the ensemble's stream, one CUDA graph per
  *   chunk of steps, so that the colonies' chains run concurrently.
  * An ensemble of up to 64 colonies that was neither tuned nor told takes LANES for
- * calls of several steps or large colonies, from the second call with the same
- * parameters on, and COOPERATIVE for the others. */
+ * calls of several steps or large colonies, after a change of parameters from the
+ * second such call on, and COOPERATIVE for the others. */
 #define SLIME_ENSEMBLE_COOPERATIVE 0u
 #define SLIME_ENSEMBLE_LANES 1u
 /* Choose the engine by hand; for LANES also the agent-kernel shape and trail

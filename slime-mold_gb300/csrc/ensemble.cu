@@ -317,7 +317,7 @@ struct slime_ensemble {
     bool last_chunk_graph = false; // the last chunk of steps replayed a graph
     int engine = SLIME_ENSEMBLE_COOPERATIVE;
     bool engine_chosen = false; // by hand, by its shape or by the autotuner; else pick_engine
-    uint64_t stable_steps = 0;  // steps made since parameters were set
+    uint64_t stable_steps = 1u << 31; // steps made since a parameter was changed
     int lane_agent_shape = 13; // agent-kernel shape of the lanes engine (persistent, texture gather)
     int lane_trail_tile = 8;   // trail tile of the lanes engine (streaming, 16-row strips)
     int max_lanes = 0;         // lanes of the lanes engine (0: one per colony, at most 64)
@@ -829,8 +829,8 @@ cudaGraphExec_t chunk_graph(slime_ensemble* e, uint32_t m) {
 // 41 / 45.  With every parameter set before each call: 16 of 256^2 208 / 398 and
 // 60 / 130, 48 of 128^2 554 / 1219 and 91 / 364.  Hence lanes for four steps a colony
 // and more at once or colonies of 100,000 agents and quarter cells on average, and
-// only where as many steps were made with these parameters before or the
-// graph is there.
+// only where the parameters are those of the creation, as many steps were made
+// with them before or the graph is there.
 void pick_engine(slime_ensemble* e, uint32_t m, bool prepared) {
     const uint64_t k = e->colonies.size();
     if (e->engine_chosen || k > kMaxLanes) return;

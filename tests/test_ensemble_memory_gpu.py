@@ -120,7 +120,7 @@ def test_steps_without_memory_for_marks(gpu, tmp_path, spare):
 S, n = {side}, {n}
 ens = sg.Ensemble([S], [S], [n], [config0_params(S, S)])
 ens.upload_agents(0, agents_uniform(n, S, S, 1.0, 2.0, seed=1))
-for m in (3, 20, 20):  # calls of a length run on lanes from the second
+for m in (3, 20, 20):
     ens.step(m)
 np.savez({str(tmp_path / "out.npz")!r}, a=ens.download_agents(0), t=ens.download_trail(0),
          marks=ens.info().marks_colonies, engine=ens.info().engine)

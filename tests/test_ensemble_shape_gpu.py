@@ -59,8 +59,7 @@ def test_the_untuned_engine_follows_the_calls(gpu):
             assert_bitexact(ens.download_trail(j), sim.download_trail(), f"trail of {j} {what}")
 
     coop, lanes = sg.ENSEMBLE_COOPERATIVE, sg.ENSEMBLE_LANES
-    step(7, coop, "the first call of a length")
-    step(7, lanes, "the second")
+    step(7, lanes, "with the parameters of the creation")
     step(2, coop, "two steps of twelve colonies")
     compare("after both engines")
     for r in range(3):
